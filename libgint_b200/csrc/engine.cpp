@@ -276,9 +276,10 @@ struct Handle {
    std::vector<SetFast> fast;
    bool basis_dirty = true, ent_dirty = true;
    // device-resident data
-   DBuf d_pool, d_ents, d_neighs, d_C0, d_C0f, d_lut, d_bw, d_ft, d_plans, d_err, d_vops;
+   DBuf d_pool, d_ents, d_neighs, d_img, d_C0, d_C0f, d_lut, d_bw, d_ft, d_plans, d_err, d_vops, d_tmap;
    DBuf d_tmax;                     // incremental replays: tile maxima of |dP|
    std::vector<VOp> vops;           // precompiled VRR instructions of all classes
+   std::vector<uint16_t> tmap;      // and the workspace elements of their targets
    std::shared_ptr<Team> team;      // device P and K (shared by the handles of an OpenMP team)
    int nspin = 0;
    size_t FP_size = 0;
@@ -413,6 +414,19 @@ static bool h2d(Handle *h, void *dst, const void *src, size_t bytes, const char 
    return ck(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream), what);
 }
 
+// The image vectors in order of their length (ties in the caller's order), for the image sums of
+// the primitive kernels: each primitive quartet tests only the images up to a length. A vector of
+// undefined length counts as the shortest, so that every primitive tests it.
+static std::vector<double4> images_by_length(const std::vector<double> &neighs) {
+   std::vector<double4> v(neighs.size() / 3);
+   for (size_t i = 0; i < v.size(); i++) {
+      const double x = neighs[3 * i], y = neighs[3 * i + 1], z = neighs[3 * i + 2], n = std::sqrt(x * x + y * y + z * z);
+      v[i] = make_double4(x, y, z, std::isnan(n) ? 0.0 : n);
+   }
+   std::stable_sort(v.begin(), v.end(), [](const double4 &a, const double4 &b) { return a.w < b.w; });
+   return v;
+}
+
 static bool upload_tables(Handle *h) {
    if (h->err) return false;
    use_device(h);
@@ -423,6 +437,8 @@ static bool upload_tables(Handle *h) {
       if (!h2d(h, h->d_plans.p, h->plans, sizeof(ClassPlan) * 256, "plans")) return false;
       if (!ensure(h, h->d_vops, h->vops.size() * sizeof(VOp), "VRR instructions")) return false;
       if (!h2d(h, h->d_vops.p, h->vops.data(), h->vops.size() * sizeof(VOp), "VRR instructions")) return false;
+      if (!ensure(h, h->d_tmap, h->tmap.size() * 2, "VRR targets")) return false;
+      if (!h2d(h, h->d_tmap.p, h->tmap.data(), h->tmap.size() * 2, "VRR targets")) return false;
       std::vector<uint8_t> lut;
       std::vector<double> bw;
       make_patch_tables(lut, bw);
@@ -489,6 +505,11 @@ static bool upload_tables(Handle *h) {
    if (h->neighs_dirty) {
       if (!ensure(h, h->d_neighs, h->neighs.size() * 8, "neighs")) return false;
       if (!h2d(h, h->d_neighs.p, h->neighs.data(), h->neighs.size() * 8, "neighs")) return false;
+      const std::vector<double4> img = images_by_length(h->neighs);
+      if (!ensure(h, h->d_img, img.size() * sizeof(double4), "neighs")) return false;
+      if (!h2d(h, h->d_img.p, img.data(), img.size() * sizeof(double4), "neighs")) return false;
+      // img goes out of scope: wait for its copy
+      if (!ck(h, cudaStreamSynchronize(h->stream), "neighs")) return false;
       h->neighs_dirty = false;
       uploaded = true;
    }
@@ -546,6 +567,7 @@ static DevCtx make_ctx(Handle *h) {
    c.pool = (const double *)h->d_pool.p;
    c.ents = (const BasisEnt *)h->d_ents.p;
    c.neighs = (const double *)h->d_neighs.p;
+   c.img = (const double4 *)h->d_img.p;
    c.Ng = h->Ng;
    c.nspin = h->nspin;
    std::memcpy(c.cell, h->cell, sizeof(c.cell));
@@ -566,6 +588,7 @@ static DevCtx make_ctx(Handle *h) {
    c.err = (int *)h->d_err.p;
    c.cnt = h->counting ? (unsigned long long *)h->d_cnt.p : nullptr;
    c.vops = (const VOp *)h->d_vops.p;
+   c.tmap = (const uint16_t *)h->d_tmap.p;
    c.gprog = group_prog(h->device);
    return c;
 }
@@ -1184,7 +1207,7 @@ void *libgint_create_handle(void) {
    for (int c = 0; c < 2 * 256; c++) h->open_of[c] = -1;
    for (int c = 0; c < 256; c++) {
       build_class_plan(c >> 6, (c >> 4) & 3, (c >> 2) & 3, c & 3, h->plans[c]);
-      build_vops(h->plans[c], h->vops);
+      build_vops(h->plans[c], h->vops, h->tmap);
       h->S_of[c] = h->plans[c].S;
       h->has_fp32[c] = class_has_fp32(c >> 6, (c >> 4) & 3, (c >> 2) & 3, c & 3);
       h->tune_prim[c] = h->tune_group[c] = 0;
@@ -1961,7 +1984,8 @@ int libgint_vrr_program(int la, int lb, int lc, int ld, void *vops, int cap, int
        !build_class_plan(la, lb, lc, ld, p))
       return -1;
    std::vector<VOp> v;
-   build_vops(p, v);
+   std::vector<uint16_t> tmap;
+   build_vops(p, v, tmap);
    if (vops) std::memcpy(vops, v.data(), sizeof(VOp) * std::min<size_t>(v.size(), (size_t)std::max(cap, 0)));
    if (info && info_cap >= 4 + 5 * p.ntg) {
       info[0] = p.V; info[1] = p.S; info[2] = p.vb[0].nm; info[3] = p.ntg;
@@ -1987,7 +2011,7 @@ void libgint_destroy_handle(void *hh) {
    }
    for (auto &rb : h->recs) { release(rb.rec); release(rb.gbuf); }
    release(h->rec_ac); release(h->rec_gscr); release(h->d_cnt);
-   DBuf *bufs[] = {&h->d_pool, &h->d_ents, &h->d_neighs, &h->d_C0, &h->d_C0f, &h->d_lut, &h->d_bw, &h->d_ft, &h->d_vops, &h->d_tmax,
+   DBuf *bufs[] = {&h->d_pool, &h->d_ents, &h->d_neighs, &h->d_img, &h->d_C0, &h->d_C0f, &h->d_lut, &h->d_bw, &h->d_ft, &h->d_vops, &h->d_tmap, &h->d_tmax,
                    &h->d_plans, &h->d_err};
    for (DBuf *b : bufs) release(*b);
    h->team.reset();

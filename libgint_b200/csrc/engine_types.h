@@ -99,6 +99,7 @@ struct ClassPlan {
    int hlev_off[kMaxLev + 1];
    int vop_off, nvop;      // the class's VRR instructions in the engine's VOp table
    int vop_lev[kMaxLev + 1];   // level l (1..nlev) is instructions [vop_lev[l-1], vop_lev[l])
+   int tmap_off;           // the class's entries in the engine's target map (build_vops)
    int want00;             // la == 0 && lc == 0: the (00|00) target collects every image
    int s00;                // offset of the (00|00) target in S (if want00)
    VBlock vb[kMaxVB];

@@ -3,12 +3,10 @@
 // Two kernels per angular-momentum class (la,lb,lc,ld), launched on class-sorted segments of
 // one batch:
 //
-//  k_prim<TS>   one team of TS lanes per primitive quartet. The lanes evaluate the images n3
-//               in parallel (truncated-Coulomb G_m by the patch Chebyshev series, or the Boys
-//               function), drop screened images, then run the Obara-Saika VRR of each
-//               surviving image cooperatively, level by level, in the team's shared-memory
-//               workspace, and sum the (e0|f0)^(0) targets over n3. The image-summed targets
-//               of the primitive go to the AC buffer.
+//  k_prim3, k_prim2   the image-summed (e0|f0)^(0) targets of every primitive quartet, into the AC
+//               buffer: truncated-Coulomb G_m by the patch Chebyshev series or the Boys function
+//               for the images that pass the truncation test, then the Obara-Saika VRR of each
+//               surviving image, generated per lane (prim3.cu) or interpreted by a team (below).
 //               (reference: src/compute_Fm.cpp:20-326, src/compute_VRR.cpp:349-458,
 //                src/compute_ECO.cpp:216-272)
 //  k_group      one warp per group (all image pairs of one set quartet for one class): for
@@ -30,95 +28,41 @@
 
 namespace gint {
 
-__constant__ int8_t c_cart_exp[8][36][3];
-__constant__ int8_t c_cart_dir[8][36];
-__constant__ int8_t c_cart_dec[8][36][3];
-__constant__ int8_t c_cart_inc[8][36][3];
 __constant__ double c_c2s[4][70];
 __constant__ double c_symm[5];
 
 static __device__ __forceinline__ int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 
-
-
 // ---------------------------------------------------------------------------------------
-// One VRR element of block b (reference VRR1..VRR6, src/compute_VRR.cpp:111-345)
-// pqz: PA[3] WP[3] QC[3] WQ[3] i2ab mrab i2cd mrcd i2z
+// k_prim2<NT>: Fm + VRR + sum over n3 for the classes without generated VRR code. One team of NT
+// threads (a warp, or a whole block) per chunk of primitive quartets:
+//  1. lane per primitive of the chunk: its geometry into shared memory;
+//  2. lane per (primitive, image) pair, over the images short enough to pass: the truncation test;
+//     passing pairs queue up in primitive order, and a batch of 32 (or the chunk's rest) goes on;
+//  3. lane per queued pair, the warps of the team sharing its orders: G_m (Chebyshev or Boys);
+//  4. the team, image after image with Fm[0] > 1e-12: the VRR as one precompiled instruction per
+//     element, level by level, and the m = 0 targets stored to (the first image of a primitive) or
+//     added to the primitive's row in AC, always by the same thread.
+// What bounds it: chains of dependent loads and FP64 operations, a batch or an image after another.
+// Chunks of up to 16 primitives fill the lanes of stages 1 to 3 (a chunk sized by the accumulators
+// of its targets held one or two primitives, and G_m ran with 3 lanes of 32); adding to AC in
+// place leaves shared memory to the workspace, so more teams are resident; each thread loads its
+// next instruction before it runs the present one. The classes of L >= 5 of the 1/4096 sample of
+// the 64-molecule l <= 3 workload: 27.4 ms before, 16.7 ms now; 2 molecules, 27 images, 27k
+// primitive quartets over 250 classes: 25.2 to 12.1 ms, kernels one after another.
 // ---------------------------------------------------------------------------------------
-template <int ST>
-static __device__ __forceinline__ void vrr_elem_s(const VBlock &b, int e, double *ws, const double *pqz) {
-   // ws element x lives at ws[x * ST]: ST = 1 for a team-shared workspace, 32 for the
-   // lane-interleaved per-lane workspaces
-   const int a = b.a, c = b.c;
-   const int na = ncart(a), nc = ncart(c);
-   const int k = e % nc, i = (e / nc) % na, mm = e / (nc * na);
-   const int m = b.lo + mm;
-   double v;
-   if (c == 0) {
-      const int d = c_cart_dir[a][i];
-      const int im = c_cart_dec[a][i][d];
-      const int na1 = ncart(a - 1);
-      const double *b1 = ws + b.in1 * ST;
-      v = pqz[d * ST] * b1[((m - b.lo1) * na1 + im) * ST] + pqz[(3 + d) * ST] * b1[((m + 1 - b.lo1) * na1 + im) * ST];
-      const int ed = c_cart_exp[a][i][d];
-      if (ed >= 2) {
-         const int iw = c_cart_dec[a - 1][im][d];
-         const int na2 = ncart(a - 2);
-         const double *b2 = ws + b.in2 * ST;
-         v += (ed - 1) * (pqz[12 * ST] * b2[((m - b.lo2) * na2 + iw) * ST] + pqz[13 * ST] * b2[((m + 1 - b.lo2) * na2 + iw) * ST]);
-      }
-   } else {
-      const int d = c_cart_dir[c][k];
-      const int km = c_cart_dec[c][k][d];
-      const int nc1 = ncart(c - 1);
-      const double *b1 = ws + b.in1 * ST;
-      v = pqz[(6 + d) * ST] * b1[(((m - b.lo1) * na + i) * nc1 + km) * ST] +
-          pqz[(9 + d) * ST] * b1[(((m + 1 - b.lo1) * na + i) * nc1 + km) * ST];
-      const int cd = c_cart_exp[c][k][d];
-      if (cd >= 2) {
-         const int kw = c_cart_dec[c - 1][km][d];
-         const int nc2 = ncart(c - 2);
-         const double *b2 = ws + b.in2 * ST;
-         v += (cd - 1) * (pqz[14 * ST] * b2[(((m - b.lo2) * na + i) * nc2 + kw) * ST] +
-                          pqz[15 * ST] * b2[(((m + 1 - b.lo2) * na + i) * nc2 + kw) * ST]);
-      }
-      if (a > 0) {
-         const int ad = c_cart_exp[a][i][d];
-         if (ad >= 1) {
-            const int im = c_cart_dec[a][i][d];
-            const double *b3 = ws + b.in3 * ST;
-            v += ad * pqz[16 * ST] * b3[(((m + 1 - b.lo3) * ncart(a - 1) + im) * nc1 + km) * ST];
-         }
-      }
-   }
-   ws[(b.off + e) * ST] = v;
+constexpr int kPrim2Chunk = 16;
+
+// the barrier of one team of NT threads
+template <int NT>
+static __device__ __forceinline__ void tsync() {
+   if constexpr (NT > 32) __syncthreads();
+   else __syncwarp();
 }
 
-// One level of the precompiled VRR (VOp, see build_vops): instructions [e0, e1) spread over the
-// lanes of a team; ws holds a zero at offset V.
-static __device__ __forceinline__ void vops_level(const VOp *__restrict__ vop, int e0, int e1, int lane, int stride,
-                                                  double *ws, const double *pqz) {
-   for (int e = e0 + lane; e < e1; e += stride) {
-      const int4 r = __ldg(reinterpret_cast<const int4 *>(vop + e));
-      VOp o;
-      memcpy(&o, &r, sizeof(VOp));
-      double v = pqz[o.zA] * ws[o.i0] + pqz[o.zA + 3] * ws[o.i1];
-      if (o.f1) v += o.f1 * (pqz[12 + 2 * o.kind] * ws[o.i2] + pqz[13 + 2 * o.kind] * ws[o.i3]);
-      if (o.f2) v += o.f2 * pqz[16] * ws[o.i4];
-      ws[o.out] = v;
-   }
-}
-
-template <int TS>
-static __device__ __forceinline__ void team_sync(unsigned mask) {
-   if (TS > 1) __syncwarp(mask);
-}
-
-// ---------------------------------------------------------------------------------------
-// k_prim: Fm + VRR + sum over n3 per primitive quartet
-// ---------------------------------------------------------------------------------------
-template <int TS>
-__global__ void __launch_bounds__(256) k_prim(DevCtx ctx, BatchArgs bt, int team_doubles) {
+template <int NT>
+__global__ void __launch_bounds__(NT == 32 ? 256 : NT, NT == 32 ? 2 : (NT == 128 ? 4 : 1))
+k_prim2(DevCtx ctx, BatchArgs bt, int cp, int team_doubles) {
    extern __shared__ __align__(16) double smem[];
    ClassPlan *pl = reinterpret_cast<ClassPlan *>(smem);
    {
@@ -129,325 +73,154 @@ __global__ void __launch_bounds__(256) k_prim(DevCtx ctx, BatchArgs bt, int team
    }
    __syncthreads();
    const int plan_doubles = (int)((sizeof(ClassPlan) + 15) / 16) * 2;
-   const int team = threadIdx.x / TS, lane = threadIdx.x % TS, nteam = blockDim.x / TS;
-   double *tws = smem + plan_doubles + (size_t)team * team_doubles;
-   const int L = pl->L, V = pl->V, S = pl->S;
-   double *ws = tws;                  // VRR workspace [V] and a zero slot
-   double *acc = tws + V + 1;         // image-summed targets [S]
-   double *pqz = acc + S;             // 17 factors of the image being processed
-   double *fmx = pqz + 17;            // per-lane Fm [TS][L+1]
-   const unsigned wl = (threadIdx.x & 31) / TS * TS;
-   const unsigned mask = (TS >= 32) ? 0xffffffffu : (((1u << TS) - 1u) << wl);
-
-   if (lane == 0) ws[V] = 0.0;
-   for (uint32_t p = blockIdx.x * nteam + team; p < bt.nprm; p += gridDim.x * nteam) {
-      PrimGeo g;
-      prim_geometry(ctx, bt.shells[bt.prm_shell[p]], bt.prm[p], g);
-      kill_if_screened(bt, bt.shells[bt.prm_shell[p]], g);
-
-      for (int j = lane; j < S; j += TS) acc[j] = 0.0;
-      double s00 = 0.0;
-      unsigned c_cheb = 0, c_boys = 0, c_vrr = 0;
-      // (ss|ss) needs no VRR: its only target is the image sum of (00|00)
-      const bool need_vrr = !(pl->want00 && pl->ntg == 1);
-      team_sync<TS>(mask);
-
-      for (int n0 = 0; n0 < ctx.Ng; n0 += TS) {
-         const int n3 = n0 + lane;
-         bool surv = false;
-         double *myfm = fmx + lane * (L + 1);
-         if (n3 < ctx.Ng && !(g.upper < 0.0)) {
-            const double T = image_T(ctx, g, n3);
-            const int br = fm_eval(ctx, L, g.R, T, g.Kfac, myfm);
-            c_cheb += (br == 1); c_boys += (br == 2);
-            s00 += myfm[0];
-            surv = need_vrr && (myfm[0] > 1.e-12);
-         }
-         unsigned bal = (TS > 1) ? ((__ballot_sync(mask, surv) & mask) >> wl) : (surv ? 1u : 0u);
-         while (bal) {
-            const int src = __ffs(bal) - 1;
-            bal &= bal - 1;
-            if (lane == src) {
-               c_vrr++;
-               const int n3s = n0 + src;
-               const double g0 = __ldg(ctx.neighs + n3s * 3 + 0), g1 = __ldg(ctx.neighs + n3s * 3 + 1),
-                            g2 = __ldg(ctx.neighs + n3s * 3 + 2);
-               const double Qp0 = g.Q[0] + g0, Qp1 = g.Q[1] + g1, Qp2 = g.Q[2] + g2;
-               const double W0 = wdist(g.zab, g.P[0], g.zcd, Qp0, g.inv_z);
-               const double W1 = wdist(g.zab, g.P[1], g.zcd, Qp1, g.inv_z);
-               const double W2 = wdist(g.zab, g.P[2], g.zcd, Qp2, g.inv_z);
-               pqz[0] = g.PA[0]; pqz[1] = g.PA[1]; pqz[2] = g.PA[2];
-               pqz[3] = W0 - g.P[0]; pqz[4] = W1 - g.P[1]; pqz[5] = W2 - g.P[2];
-               pqz[6] = g.QC[0]; pqz[7] = g.QC[1]; pqz[8] = g.QC[2];
-               pqz[9] = W0 - Qp0; pqz[10] = W1 - Qp1; pqz[11] = W2 - Qp2;
-               pqz[12] = g.i2ab; pqz[13] = g.mrab; pqz[14] = g.i2cd; pqz[15] = g.mrcd; pqz[16] = g.i2z;
-               const int n00 = pl->vb[0].nm;
-               for (int q = 0; q < n00; q++) ws[q] = myfm[q];
-            }
-            team_sync<TS>(mask);
-            for (int lv = 1; lv <= pl->nlev; lv++) {
-               vops_level(ctx.vops + pl->vop_off, pl->vop_lev[lv - 1], pl->vop_lev[lv], lane, TS, ws, pqz);
-               team_sync<TS>(mask);
-            }
-            for (int t = 0; t < pl->ntg; t++) {
-               if (pl->want00 && pl->tg_e[t] == 0 && pl->tg_f[t] == 0) continue;
-               const double *srcp = ws + pl->tg_voff[t];
-               double *dst = acc + pl->tg_soff[t];
-               for (int q = lane; q < pl->tg_n[t]; q += TS) dst[q] += srcp[q];
-            }
-            team_sync<TS>(mask);
-         }
-      }
-      if (pl->want00) {
-         if (TS > 1) {
-#pragma unroll
-            for (int o = TS / 2; o > 0; o >>= 1) s00 += __shfl_down_sync(mask, s00, o, TS);
-         }
-         if (lane == 0) acc[pl->s00] += s00;
-      }
-      if (ctx.cnt) {
-         if (TS > 1) {
-#pragma unroll
-            for (int o = TS / 2; o > 0; o >>= 1) {
-               c_cheb += __shfl_down_sync(mask, c_cheb, o, TS);
-               c_boys += __shfl_down_sync(mask, c_boys, o, TS);
-               c_vrr += __shfl_down_sync(mask, c_vrr, o, TS);
-            }
-         }
-         if (lane == 0) {
-            atomicAdd(ctx.cnt + bt.cls * 4 + 0, (unsigned long long)c_cheb);
-            atomicAdd(ctx.cnt + bt.cls * 4 + 1, (unsigned long long)c_boys);
-            atomicAdd(ctx.cnt + bt.cls * 4 + 2, (unsigned long long)c_vrr);
-            atomicAdd(ctx.cnt + bt.cls * 4 + 3, 1ull);
-         }
-      }
-      team_sync<TS>(mask);
-      double *out = bt.AC + (size_t)p * S;
-      for (int j = lane; j < S; j += TS) out[j] = acc[j];
-      team_sync<TS>(mask);
-   }
-}
-
-// ---------------------------------------------------------------------------------------
-// k_prim2<LANE_VRR>: Fm + VRR + sum over n3, one warp per chunk of primitive quartets with
-// two compaction stages. (1) all (primitive, image) pairs get the cheap truncation test
-// T <= R^2 + 11R + 50 and the passing pairs are queued; (2) the queue is evaluated 32 at a time
-// (G_m by the Chebyshev series or Boys) so that every lane does useful work, and the images with
-// Fm[0] > 1e-12 are queued again; (3) their VRR runs one image per lane (LANE_VRR, small
-// classes, lane-interleaved workspaces) or one image per warp (level-parallel), and the m = 0
-// targets are summed per primitive in shared memory.
-// ---------------------------------------------------------------------------------------
-template <bool LANE_VRR>
-__global__ void __launch_bounds__(256) k_prim2(DevCtx ctx, BatchArgs bt, int cp, int warp_doubles) {
-   extern __shared__ __align__(16) double smem[];
-   ClassPlan *pl = reinterpret_cast<ClassPlan *>(smem);
-   {
-      const int nwords = (int)(sizeof(ClassPlan) / 4);
-      const int *src = reinterpret_cast<const int *>(bt.plan);
-      int *dst = reinterpret_cast<int *>(smem);
-      for (int w = threadIdx.x; w < nwords; w += blockDim.x) dst[w] = src[w];
-   }
-   __syncthreads();
-   const int plan_doubles = (int)((sizeof(ClassPlan) + 15) / 16) * 2;
-   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
-   double *wb = smem + plan_doubles + (size_t)warp * warp_doubles;
-   const int L = pl->L, S = pl->S, Ng = ctx.Ng;
-   const int LF = L + 1;
-   // per-warp layout
-   PrimGeo *geo = reinterpret_cast<PrimGeo *>(wb);                     // [cp]
-   double *s00 = wb + cp * (sizeof(PrimGeo) / 8);                     // [cp]
-   double *acc = s00 + cp;                                            // [cp][S]
-   int *q1i = reinterpret_cast<int *>(acc + (size_t)cp * S);          // [64] pair index
-   double *q1t = acc + (size_t)cp * S + 32;                           // [64] T
-   int *q2i = reinterpret_cast<int *>(q1t + 64);                      // [64] pair index
-   double *q2f = q1t + 64 + 32;                                       // [64][LF] Fm
-   double *pqz = q2f + 64 * LF;                                       // [17][32] (lane) or [17]
-   double *ws = pqz + (LANE_VRR ? 17 * 32 : 18);                      // [V][32] (lane) or [V] + zero
-   const bool need_vrr = !(pl->want00 && pl->ntg == 1);
+   const int team = threadIdx.x / NT, tl = threadIdx.x % NT, lane = threadIdx.x & 31, tw = tl >> 5;
+   const int nteam = blockDim.x / NT;
+   double *tb = smem + plan_doubles + (size_t)team * team_doubles;
+   const int L = pl->L, S = pl->S, Ng = ctx.Ng, LF = L + 1;
+   // per-team layout (prim2_team_doubles)
+   PrimGeo *geo = reinterpret_cast<PrimGeo *>(tb);                     // [cp]
+   double *s00 = tb + cp * (int)(sizeof(PrimGeo) / 8);                 // [cp]
+   double *q1t = s00 + cp;                                            // [64] T of the queued pairs
+   int *q1i = reinterpret_cast<int *>(q1t + 64);                      // [64] primitive << 8 | image
+   double *q2f = q1t + 64 + 32;                                       // [32][LF] Fm of the batch
+   double *pqz = q2f + 32 * LF;                                       // [18] factors of one image
+   double *ws = pqz + 18;                                             // [V] VRR workspace and a zero
+   const bool want00 = pl->want00 != 0, need_vrr = !(want00 && pl->ntg == 1);
+   const int s00_at = want00 ? pl->s00 : -1;
    const unsigned below = (1u << lane) - 1u;
+   const int4 *vop = reinterpret_cast<const int4 *>(ctx.vops + pl->vop_off);
+   const uint16_t *tmap = ctx.tmap + pl->tmap_off;
+   const int nvop = pl->nvop, nlev = pl->nlev;
    unsigned long long c_cheb = 0, c_boys = 0, c_vrr = 0;
-   if (!LANE_VRR && lane == 0) ws[pl->V] = 0.0;
+   if (tl == 0) ws[pl->V] = 0.0;
 
    const uint32_t nchunk = (bt.nprm + cp - 1) / cp;
-   for (uint32_t ch = blockIdx.x * nwarp + warp; ch < nchunk; ch += gridDim.x * nwarp) {
+   for (uint32_t ch = blockIdx.x * nteam + team; ch < nchunk; ch += gridDim.x * nteam) {
       const uint32_t p0 = ch * cp;
       const int np = (int)min((uint32_t)cp, bt.nprm - p0);
-      // ---- per-primitive geometry (reference src/compute_Fm.cpp:66-159, :202-210, :281-290)
-      if (lane < np) {
-         const uint32_t p = p0 + lane;
+      // every warp of the team numbers and tests the pairs for itself, from the geometry of warp 0
+      tsync<NT>();
+      if (tw == 0 && lane < np) {
          PrimGeo g;
-         prim_geometry(ctx, bt.shells[bt.prm_shell[p]], bt.prm[p], g);
-         kill_if_screened(bt, bt.shells[bt.prm_shell[p]], g);
+         const ShellRec sh = bt.shells[bt.prm_shell[p0 + lane]];
+         prim_geometry(ctx, sh, bt.prm[p0 + lane], g);
+         kill_if_screened(bt, sh, g);
          geo[lane] = g;
          s00[lane] = 0.0;
       }
-      for (int j = lane; j < np * S; j += 32) acc[j] = 0.0;
-      __syncwarp();
-
-      int n1 = 0, n2 = 0;
-      const int npair = np * Ng;
-      // stage 3: VRR of the queued images [0, cnt)
-      auto run_vrr = [&](int cnt) {
-         if (LANE_VRR) {
-            if (lane < cnt) {
-               const int pi = q2i[lane];
-               const int p = pi / Ng, n3 = pi - p * Ng;
-               const PrimGeo &g = geo[p];
-               const double g0 = __ldg(ctx.neighs + n3 * 3 + 0), g1 = __ldg(ctx.neighs + n3 * 3 + 1),
-                            g2 = __ldg(ctx.neighs + n3 * 3 + 2);
-               const double Qp[3] = {g.Q[0] + g0, g.Q[1] + g1, g.Q[2] + g2};
-               double *pz = pqz + lane;
-               for (int q = 0; q < 3; q++) {
-                  const double W = wdist(g.zab, g.P[q], g.zcd, Qp[q], g.inv_z);
-                  pz[q * 32] = g.PA[q];
-                  pz[(3 + q) * 32] = W - g.P[q];
-                  pz[(6 + q) * 32] = g.QC[q];
-                  pz[(9 + q) * 32] = W - Qp[q];
-               }
-               pz[12 * 32] = g.i2ab; pz[13 * 32] = g.mrab; pz[14 * 32] = g.i2cd; pz[15 * 32] = g.mrcd;
-               pz[16 * 32] = g.i2z;
-               double *w = ws + lane;
-               const int n00 = pl->vb[0].nm;
-               for (int q = 0; q < n00; q++) w[q * 32] = q2f[lane * LF + q];
-               for (int bb = 1; bb < pl->nvb; bb++) {
-                  const VBlock vb = pl->vb[bb];
-                  for (int e = 0; e < vb.nelem; e++) vrr_elem_s<32>(vb, e, w, pz);
-               }
-               double *ap = acc + (size_t)p * S;
-               for (int t = 0; t < pl->ntg; t++) {
-                  if (pl->want00 && pl->tg_e[t] == 0 && pl->tg_f[t] == 0) continue;
-                  const double *sp = w + pl->tg_voff[t] * 32;
-                  double *dp = ap + pl->tg_soff[t];
-                  for (int q = 0; q < pl->tg_n[t]; q++) atomicAdd(dp + q, sp[q * 32]);
-               }
-            }
-            __syncwarp();
-         } else {
-            for (int s = 0; s < cnt; s++) {
-               const int pi = q2i[s];
-               const int p = pi / Ng, n3 = pi - p * Ng;
-               const PrimGeo &g = geo[p];
-               if (lane < 3) {
-                  const int q = lane;
-                  const double gq = __ldg(ctx.neighs + n3 * 3 + q);
-                  const double Qp = g.Q[q] + gq;
-                  const double W = wdist(g.zab, g.P[q], g.zcd, Qp, g.inv_z);
-                  pqz[q] = g.PA[q]; pqz[3 + q] = W - g.P[q]; pqz[6 + q] = g.QC[q]; pqz[9 + q] = W - Qp;
-               } else if (lane == 3) {
-                  pqz[12] = g.i2ab; pqz[13] = g.mrab; pqz[14] = g.i2cd; pqz[15] = g.mrcd; pqz[16] = g.i2z;
-               }
-               const int n00 = pl->vb[0].nm;
-               for (int q = lane; q < n00; q += 32) ws[q] = q2f[s * LF + q];
-               __syncwarp();
-               for (int lv = 1; lv <= pl->nlev; lv++) {
-                  vops_level(ctx.vops + pl->vop_off, pl->vop_lev[lv - 1], pl->vop_lev[lv], lane, 32, ws, pqz);
-                  __syncwarp();
-               }
-               double *ap = acc + (size_t)p * S;
-               for (int t = 0; t < pl->ntg; t++) {
-                  if (pl->want00 && pl->tg_e[t] == 0 && pl->tg_f[t] == 0) continue;
-                  const double *sp = ws + pl->tg_voff[t];
-                  double *dp = ap + pl->tg_soff[t];
-                  for (int q = lane; q < pl->tg_n[t]; q += 32) dp[q] += sp[q];
-               }
-               __syncwarp();
-            }
-         }
-      };
-      // stage 2: G_m of the queued pairs [0, cnt), one per lane
-      auto run_fm = [&](int cnt) {
-         bool surv = false;
-         double fm[kMaxLL + 1];
-         int pi = 0;
+      tsync<NT>();
+      int start;
+      const int npair = pair_starts(lane < np ? image_count(ctx.img, Ng, geo[lane]) : 0, np, lane, start);
+      double *out = bt.AC + (size_t)p0 * S;
+      unsigned done = 0;   // primitives whose row holds an image already
+      // stages 3 and 4 of the queued pairs [0, cnt)
+      auto run_batch = [&](int cnt) {
          if (lane < cnt) {
-            pi = q1i[lane];
-            const double T = q1t[lane];
-            const int p = pi / Ng;
+            const int pk = q1i[lane];
+            const int br = fm_eval_geo<-1>(ctx, L, geo[pk >> 8], q1t[lane], q2f + lane * LF, tw, NT / 32);
+            if (tw == 0) { c_cheb += (br == 1); c_boys += (br == 2); }
+         }
+         tsync<NT>();
+         const double f0 = lane < cnt ? q2f[lane * LF] : 0.0;
+         if (want00 && tw == 0) {
+            const int p = lane < cnt ? q1i[lane] >> 8 : -1 - lane;
+            SegSum<double> sg = make_segsum<double>(p, lane, s00 + max(p, 0));
+            sg(0, f0);
+         }
+         unsigned bal = __ballot_sync(0xffffffffu, need_vrr && lane < cnt && f0 > 1.e-12);
+         if (tl == 0) c_vrr += __popc(bal);
+         for (; bal; bal &= bal - 1) {
+            const int s = __ffs(bal) - 1, pk = q1i[s], p = pk >> 8;
             const PrimGeo &g = geo[p];
-            const int br = fm_eval(ctx, L, g.R, T, g.Kfac, fm);
-            c_cheb += (br == 1); c_boys += (br == 2);
-            if (pl->want00) atomicAdd(s00 + p, fm[0]);
-            surv = need_vrr && (fm[0] > 1.e-12);
-         }
-         const unsigned bal = __ballot_sync(0xffffffffu, surv);
-         if (surv) {
-            const int pos = n2 + __popc(bal & below);
-            q2i[pos] = pi;
-            for (int q = 0; q < LF; q++) q2f[pos * LF + q] = fm[q];
-         }
-         n2 += __popc(bal);
-         __syncwarp();
-         const int step = LANE_VRR ? 32 : 1;
-         while (n2 >= step || (n2 > 0 && !LANE_VRR)) {
-            const int cnt2 = LANE_VRR ? 32 : n2;
-            c_vrr += (lane == 0) ? cnt2 : 0;
-            run_vrr(cnt2);
-            // shift the remainder down
-            const int rem = n2 - cnt2;
-            int v = 0;
-            double tmp[kMaxLL + 1];
-            if (lane < rem) {
-               v = q2i[cnt2 + lane];
-               for (int q = 0; q < LF; q++) tmp[q] = q2f[(cnt2 + lane) * LF + q];
+            if (tl < 3) {
+               const double Qp = g.Q[tl] + __ldg(reinterpret_cast<const double *>(ctx.img + (pk & 255)) + tl);
+               const double W = wdist(g.zab, g.P[tl], g.zcd, Qp, g.inv_z);
+               pqz[tl] = g.PA[tl]; pqz[3 + tl] = W - g.P[tl]; pqz[6 + tl] = g.QC[tl]; pqz[9 + tl] = W - Qp;
+            } else if (tl == 3) {
+               pqz[12] = g.i2ab; pqz[13] = g.mrab; pqz[14] = g.i2cd; pqz[15] = g.mrcd; pqz[16] = g.i2z;
             }
-            __syncwarp();
-            if (lane < rem) {
-               q2i[lane] = v;
-               for (int q = 0; q < LF; q++) q2f[lane * LF + q] = tmp[q];
+            if (tl < LF) ws[tl] = q2f[s * LF + tl];   // (0|0)^(m), m = 0..L
+            int4 next = __ldg(vop + min(tl, nvop - 1));
+            tsync<NT>();
+            int e0 = 0;
+            for (int lv = 1; lv <= nlev; lv++) {
+               const int e1 = pl->vop_lev[lv];
+               for (int e = e0 + tl; e < e1; e += NT) {
+                  VOp o;
+                  memcpy(&o, &next, sizeof(VOp));
+                  const int en = e + NT < e1 ? e + NT : e1 + tl;
+                  next = __ldg(vop + min(en, nvop - 1));
+                  double v = pqz[o.zA] * ws[o.i0] + pqz[o.zA + 3] * ws[o.i1];
+                  if (o.f1) v += o.f1 * (pqz[12 + 2 * o.kind] * ws[o.i2] + pqz[13 + 2 * o.kind] * ws[o.i3]);
+                  if (o.f2) v += o.f2 * pqz[16] * ws[o.i4];
+                  ws[o.out] = v;
+               }
+               if (e0 + tl >= e1) next = __ldg(vop + min(e1 + tl, nvop - 1));   // idle on this level
+               e0 = e1;
+               tsync<NT>();
             }
-            __syncwarp();
-            n2 = rem;
+            double *row = out + (size_t)p * S;
+            if (done >> p & 1) {
+               for (int j = tl; j < S; j += NT)
+                  if (j != s00_at) row[j] += ws[__ldg(tmap + j)];
+            } else {
+               for (int j = tl; j < S; j += NT)
+                  if (j != s00_at) row[j] = ws[__ldg(tmap + j)];
+            }
+            done |= 1u << p;
+            tsync<NT>();
          }
       };
-      // stage 1: truncation test over all (primitive, image) pairs
+      // stage 2
+      int n1 = 0;
       for (int b0 = 0; b0 < npair; b0 += 32) {
-         const int pi = b0 + lane;
          bool pass = false;
          double T = 0.0;
-         if (pi < npair) {
-            const int p = pi / Ng, n3 = pi - p * Ng;
-            const PrimGeo &g = geo[p];
-            T = image_T(ctx, g, n3);
-            pass = !(T > g.upper);   // g.upper = trunc_upper(g.R), or -1 for a screened primitive
+         int tn;
+         const int tp = pair_prim(b0, start, lane, tn);
+         if (b0 + lane < npair) {
+            const PrimGeo &g = geo[tp];
+            const double *im = reinterpret_cast<const double *>(ctx.img + tn);
+            const double d0 = rsub(g.D[0], __ldg(im)), d1 = rsub(g.D[1], __ldg(im + 1)), d2 = rsub(g.D[2], __ldg(im + 2));
+            T = rmul(g.rho, rdot3(d0, d0, d1, d1, d2, d2));
+            pass = !(T > g.upper);
          }
          const unsigned bal = __ballot_sync(0xffffffffu, pass);
-         if (pass) {
+         if (pass && tw == 0) {
             const int pos = n1 + __popc(bal & below);
-            q1i[pos] = pi;
+            q1i[pos] = (tp << 8) | tn;
             q1t[pos] = T;
          }
          n1 += __popc(bal);
-         __syncwarp();
+         tsync<NT>();
          if (n1 >= 32) {
-            run_fm(32);
+            run_batch(32);
             const int rem = n1 - 32;
-            int vi = 0; double vt = 0.0;
-            if (lane < rem) { vi = q1i[32 + lane]; vt = q1t[32 + lane]; }
-            __syncwarp();
-            if (lane < rem) { q1i[lane] = vi; q1t[lane] = vt; }
-            __syncwarp();
+            int vi = 0;
+            double vt = 0.0;
+            tsync<NT>();
+            if (tw == 0 && lane < rem) { vi = q1i[32 + lane]; vt = q1t[32 + lane]; }
+            tsync<NT>();
+            if (tw == 0 && lane < rem) { q1i[lane] = vi; q1t[lane] = vt; }
+            tsync<NT>();
             n1 = rem;
          }
       }
-      if (n1 > 0) { run_fm(n1); n1 = 0; }
-      if (n2 > 0) {
-         c_vrr += (lane == 0) ? n2 : 0;
-         run_vrr(n2);
-         n2 = 0;
-      }
-      // the (00|00) target collects every image (reference src/compute_VRR.cpp:381-389)
-      if (pl->want00 && lane < np) acc[(size_t)lane * S + pl->s00] += s00[lane];
-      if (lane == 0 && ctx.cnt) atomicAdd(ctx.cnt + bt.cls * 4 + 3, (unsigned long long)np);
-      __syncwarp();
-      double *out = bt.AC + (size_t)p0 * S;
-      for (int j = lane; j < np * S; j += 32) out[j] = acc[j];
-      __syncwarp();
+      if (n1 > 0) run_batch(n1);
+      // the rows without an image, and the (00|00) target, which collects every image's Fm[0]
+      // (reference src/compute_VRR.cpp:381-389)
+      tsync<NT>();
+      for (int p = 0; p < np; p++)
+         if (!(done >> p & 1))
+            for (int j = tl; j < S; j += NT)
+               if (j != s00_at) out[(size_t)p * S + j] = 0.0;
+      if (want00 && tl < np) out[(size_t)tl * S + s00_at] = s00[tl];
+      if (tl == 0 && ctx.cnt) atomicAdd(ctx.cnt + bt.cls * 4 + 3, (unsigned long long)np);
    }
-   if (ctx.cnt) {
+   if (ctx.cnt && tw == 0) {
       for (int o = 16; o > 0; o >>= 1) {
          c_cheb += __shfl_down_sync(0xffffffffu, c_cheb, o);
          c_boys += __shfl_down_sync(0xffffffffu, c_boys, o);
-         c_vrr += __shfl_down_sync(0xffffffffu, c_vrr, o);
       }
       if (lane == 0) {
          atomicAdd(ctx.cnt + bt.cls * 4 + 0, c_cheb);
@@ -869,13 +642,7 @@ cudaError_t upload_constant_tables(const double *c2s_l0to3, const double *symm5)
          for (int k = 0; k < nk; k++)
             if (((c2s_mask(l, m) >> k & 1) != 0) != (c2s_l0to3[l * 70 + m * nk + k] != 0.0)) return cudaErrorInvalidValue;
    }
-   CartTables t;
-   make_cart_tables(t);
    cudaError_t err;
-   if ((err = cudaMemcpyToSymbol(c_cart_exp, t.exp_, sizeof(t.exp_))) != cudaSuccess) return err;
-   if ((err = cudaMemcpyToSymbol(c_cart_dir, t.dir, sizeof(t.dir))) != cudaSuccess) return err;
-   if ((err = cudaMemcpyToSymbol(c_cart_dec, t.dec, sizeof(t.dec))) != cudaSuccess) return err;
-   if ((err = cudaMemcpyToSymbol(c_cart_inc, t.inc, sizeof(t.inc))) != cudaSuccess) return err;
    if ((err = cudaMemcpyToSymbol(c_c2s, c2s_l0to3, sizeof(double) * 4 * 70)) != cudaSuccess) return err;
    return cudaMemcpyToSymbol(c_symm, symm5, sizeof(double) * 5);
 }
@@ -894,23 +661,6 @@ static int max_dyn_smem() {
    return smax;
 }
 
-template <int TS>
-static cudaError_t launch_prim_t(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan &hp, cudaStream_t st) {
-   const int L = hp.L;
-   int team_doubles = hp.V + 1 + hp.S + 17 + TS * (L + 1);
-   team_doubles = (team_doubles + 1) & ~1;
-   const int budget = std::min(max_dyn_smem(), 200 * 1024);
-   const size_t plan_bytes = (size_t)plan_smem_doubles() * 8;
-   int teams = (int)((budget - (int)plan_bytes) / ((size_t)team_doubles * 8));
-   teams = std::min(teams, 256 / TS);
-   if (teams < 1) return cudaErrorInvalidConfiguration;
-   const size_t smem = plan_bytes + (size_t)teams * team_doubles * 8;
-   long blocks = ((long)bt.nprm + teams - 1) / teams;
-   blocks = std::max(1L, std::min(blocks, 148L * 64));
-   k_prim<TS><<<(unsigned)blocks, teams * TS, smem, st>>>(ctx, bt, team_doubles);
-   return cudaGetLastError();
-}
-
 int prim_team_size(const ClassPlan &hp) {
    const int w = hp.V + hp.S;
    if (w <= 40) return 1;
@@ -919,23 +669,21 @@ int prim_team_size(const ClassPlan &hp) {
    return 32;
 }
 
-// k_prim2 launch shape: primitives per warp chunk and the per-warp shared-memory size. The chunk's
-// image-summed targets (cp x S doubles) are the largest part of a warp's shared memory, and
-// shared memory bounds the warps per SM of the large classes, so a chunk holds about 512 targets.
-static void prim2_shape(const ClassPlan &hp, bool lane_vrr, int *cp, size_t *warp_doubles) {
-   int c = std::max(1, std::min(32, 512 / std::max(1, hp.S)));
-   const size_t geo = (sizeof(PrimGeo) / 8);
-   size_t w = geo * c + c + (size_t)c * hp.S + 32 + 64 + 32 + 64 * (size_t)(hp.L + 1) +
-              (lane_vrr ? 17 * 32 + 32 * (size_t)hp.V : 18 + (size_t)hp.V + 2);
-   *cp = c;
-   *warp_doubles = (w + 1) & ~(size_t)1;
+// shared memory of one k_prim2 team, in doubles: cp geometries and (00|00) sums, the pair queue, one
+// batch's Fm, one image's factors and the VRR workspace with its zero
+static size_t prim2_team_doubles(const ClassPlan &hp, int cp) {
+   const size_t w = (size_t)cp * (sizeof(PrimGeo) / 8 + 1) + 64 + 32 + 32 * (size_t)(hp.L + 1) + 18 + (size_t)hp.V + 1;
+   return (w + 1) & ~(size_t)1;
 }
 
-static bool prim2_lane(const ClassPlan &hp) { return hp.V <= 96; }
+// A workspace of this many doubles is worked on by a block instead of a warp: a warp takes a level of
+// it in many rounds, and too few warps fit an SM to hide them.
+constexpr int kPrim2BlockDoubles = 1500;
+constexpr int kPrim2WideDoubles = 5000;    // and by 256 threads instead of 128 from here on
 
-
-// Primitive-kernel choice: k_prim3 (generated VRR) for the classes it covers, then k_prim2,
-// then the team kernel for the largest classes.
+// Primitive-kernel choice: k_prim3 (generated VRR) for the classes it covers, else k_prim2. Its
+// team is a warp for small workspaces and a block for large ones, and for segments whose chunks are
+// fewer than would give every SM four warps (there one image's chain of levels is the whole time).
 cudaError_t launch_prim(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan &hp, cudaStream_t st) {
    if (bt.nprm == 0) return cudaSuccess;
    if (bt.prim_variant == 0 || bt.fp32) {
@@ -943,34 +691,29 @@ cudaError_t launch_prim(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan 
       if (prim3_launch(ctx, bt, st, &err)) return err;
    }
    if (bt.fp32) return cudaErrorInvalidValue;   // FP32 segments exist only for classes with k_prim3
-   {
-      const bool lane = prim2_lane(hp);
-      int cp = 1;
-      size_t wd = 0;
-      prim2_shape(hp, lane, &cp, &wd);
-      const int budget = std::min(max_dyn_smem(), 200 * 1024);
-      const size_t plan_bytes = (size_t)plan_smem_doubles() * 8;
-      int nw = (int)((budget - (int)plan_bytes) / (wd * 8));
-      nw = std::min(nw, 8);
-      if (nw >= 1) {
-         const size_t smem = plan_bytes + (size_t)nw * wd * 8;
-         const long nchunk = ((long)bt.nprm + cp - 1) / cp;
-         long blocks = std::max(1L, std::min((nchunk + nw - 1) / nw, 148L * 32));
-         if (lane) {
-            k_prim2<true><<<(unsigned)blocks, nw * 32, smem, st>>>(ctx, bt, cp, (int)wd);
-         } else {
-            k_prim2<false><<<(unsigned)blocks, nw * 32, smem, st>>>(ctx, bt, cp, (int)wd);
-         }
-         return cudaGetLastError();
-      }
-      // the largest classes fall through to the team kernel
+   // a chunk is as large as gives every resident team one, within what fills a G_m batch (about four
+   // pairs a primitive with images, one without) and kPrim2Chunk; where the VRR is the larger part
+   // of a primitive's time the lanes of G_m matter less than a finer split
+   const int fill = (hp.V >= 1000 ? 2 : 4) * (ctx.Ng == 1 ? 2 : 1);
+   auto chunk = [&](long teams) { return (int)std::max((long)fill, std::min((long)kPrim2Chunk, ((long)bt.nprm + teams - 1) / teams)); };
+   const size_t plan_bytes = (size_t)plan_smem_doubles() * 8;
+   int cp = chunk(148 * 14);
+   long nchunk = ((long)bt.nprm + cp - 1) / cp;
+   if (hp.V >= kPrim2BlockDoubles || (hp.V >= 128 && nchunk < 148 * 4)) {
+      cp = chunk(148 * 4);
+      nchunk = ((long)bt.nprm + cp - 1) / cp;
+      const size_t wd = prim2_team_doubles(hp, cp), smem = plan_bytes + wd * 8;
+      const unsigned blocks = (unsigned)std::min(nchunk, 148L * 64);
+      if (hp.V >= kPrim2WideDoubles) k_prim2<256><<<blocks, 256, smem, st>>>(ctx, bt, cp, (int)wd);
+      else k_prim2<128><<<blocks, 128, smem, st>>>(ctx, bt, cp, (int)wd);
+      return cudaGetLastError();
    }
-   switch (prim_team_size(hp)) {
-      case 1: return launch_prim_t<1>(ctx, bt, hp, st);
-      case 4: return launch_prim_t<4>(ctx, bt, hp, st);
-      case 8: return launch_prim_t<8>(ctx, bt, hp, st);
-      default: return launch_prim_t<32>(ctx, bt, hp, st);
-   }
+   const size_t wd = prim2_team_doubles(hp, cp);
+   const int nwmax = std::max(1, std::min(8, (int)((112 * 1024 - plan_bytes) / (wd * 8))));   // two blocks per SM
+   const int nw = (int)std::max(1L, std::min((long)nwmax, (nchunk + 147) / 148));
+   const unsigned blocks = (unsigned)std::max(1L, std::min((nchunk + nw - 1) / nw, 148L * 64));
+   k_prim2<32><<<blocks, nw * 32, plan_bytes + (size_t)nw * wd * 8, st>>>(ctx, bt, cp, (int)wd);
+   return cudaGetLastError();
 }
 
 size_t group_warp_doubles(const ClassPlan &hp) {
@@ -1263,8 +1006,7 @@ const uint2 *group_prog(int device) {
 cudaError_t preload_kernels() {
    cudaError_t e;
    const int smax = max_dyn_smem();
-   const void *fns[] = {(const void *)k_prim<1>, (const void *)k_prim<4>, (const void *)k_prim<8>,
-                        (const void *)k_prim<32>, (const void *)k_prim2<true>, (const void *)k_prim2<false>,
+   const void *fns[] = {(const void *)k_prim2<32>, (const void *)k_prim2<128>, (const void *)k_prim2<256>,
                         (const void *)k_group, (const void *)k_group_lane, (const void *)k_group_block<128>,
                         (const void *)k_group_block<256>};
    for (const void *f : fns)

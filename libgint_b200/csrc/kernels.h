@@ -17,6 +17,7 @@ struct DevCtx {
    const double *pool;        // exponents and normalised coefficients
    const BasisEnt *ents;
    const double *neighs;      // Ng lattice vectors
+   const double4 *img;        // the same in order of their length: {vector, length}
    int Ng;
    int nspin;
    double cell[18];           // h (rows = lattice vectors) and h^-1
@@ -34,6 +35,7 @@ struct DevCtx {
    int *err;
    unsigned long long *cnt;   // optional event counters per class [256][4], or null
    const VOp *vops;           // precompiled VRR instructions of every class (build_vops)
+   const uint16_t *tmap;      // VRR workspace element of every contracted target of every class (build_vops)
    const uint2 *gprog;        // HRR instructions of every class (group_prog), shared by all handles
 };
 
@@ -61,12 +63,12 @@ struct BatchArgs {
    int fp32;                  // 1: the segment's shell quartets run in FP32 (Fm, VRR, contraction, HRR)
    double *gscratch;          // HRR workspace in global memory for the largest classes
    int cls;                   // la*64 + lb*16 + lc*4 + ld
-   int prim_variant;          // 0: k_prim3 where the class has it (lane per image); 1: k_prim2 (warp per image)
+   int prim_variant;          // 0: k_prim3 where the class has it (lane per image); 1: k_prim2 (team per image)
    int group_variant;         // 0: k_group3 where the class has it (lane per row); 1: k_group (warp per row)
 };
 
 bool build_class_plan(int la, int lb, int lc, int ld, ClassPlan &p);
-void build_vops(ClassPlan &p, std::vector<VOp> &out);
+void build_vops(ClassPlan &p, std::vector<VOp> &out, std::vector<uint16_t> &tmap);
 cudaError_t upload_constant_tables(const double *c2s_l0to3, const double *symm5);
 cudaError_t launch_prim(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan &hp, cudaStream_t st);
 cudaError_t launch_group(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan &hp, cudaStream_t st);

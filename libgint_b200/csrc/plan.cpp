@@ -149,8 +149,9 @@ static int lowered_idx(const int e[3], int d, int n) { int f[3] = {e[0], e[1], e
 
 // Appends the VRR of class p as one instruction per workspace element, level by level, with the
 // same inputs and multipliers as the element formulas of the interpreted kernels
-// (reference VRR1..VRR6, src/compute_VRR.cpp:111-345), and records the level boundaries.
-void build_vops(ClassPlan &p, std::vector<VOp> &out) {
+// (reference VRR1..VRR6, src/compute_VRR.cpp:111-345), and records the level boundaries; and
+// appends to tmap the workspace element of every contracted target.
+void build_vops(ClassPlan &p, std::vector<VOp> &out, std::vector<uint16_t> &tmap) {
    const int16_t zero = (int16_t)p.V;   // the workspace's zero slot
    p.vop_off = (int)out.size();
    p.vop_lev[0] = 0;
@@ -202,6 +203,10 @@ void build_vops(ClassPlan &p, std::vector<VOp> &out) {
       p.vop_lev[lv] = (int)out.size() - p.vop_off;
    }
    p.nvop = (int)out.size() - p.vop_off;
+   p.tmap_off = (int)tmap.size();
+   tmap.resize(tmap.size() + p.S);
+   for (int t = 0; t < p.ntg; t++)
+      for (int q = 0; q < p.tg_n[t]; q++) tmap[p.tmap_off + p.tg_soff[t] + q] = (uint16_t)(p.tg_voff[t] + q);
 }
 
 }  // namespace gint

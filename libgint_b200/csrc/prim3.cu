@@ -4,8 +4,8 @@
 // One warp owns a chunk of CP primitive quartets (reference src/compute_Fm.cpp:20-326,
 // src/compute_VRR.cpp:349-458, src/compute_ECO.cpp:216-272):
 //  1. lane per primitive: the geometry (P, Q, the minimum-image shift, Kfac, R) into shared;
-//  2. lane per (primitive, image) pair: the truncation test T <= R^2 + 11 R + 50; passing
-//     pairs are compacted into a queue;
+//  2. lane per (primitive, image) pair, over the images short enough to pass (image_count): the
+//     truncation test T <= R^2 + 11 R + 50; passing pairs are compacted into a queue;
 //  3. lane per queued pair: G_m (Chebyshev patch series or Boys); pairs with Fm[0] > 1e-12 are
 //     compacted into a second queue; when la = lc = 0 every pair's Fm[0] goes to the (00|00)
 //     target, screened or not, as in the reference;
@@ -51,43 +51,11 @@ struct Prim3Shape {
    static constexpr int THREADS = MINB == 3 ? 192 : 256;
 };
 
-// Segmented sum over adjacent lanes that carry the same key (keys are contiguous runs); the
-// first lane of each run adds the run's sum to dst[s]. R = double, or float on the FP32 path.
-template <class R>
-struct SegSum {
-   unsigned same;   // bit o: lane + 2^o carries this lane's key
-   bool head;
-   R *dst;
-   __device__ __forceinline__ void operator()(int s, R v) {
-#pragma unroll
-      for (int o = 0; o < 5; o++) {
-         const R u = __shfl_down_sync(kFull, v, 1 << o);
-         if (same & (1u << o)) v += u;
-      }
-      if (head) dst[s] += v;
-   }
-};
-
-template <class R>
-static __device__ __forceinline__ SegSum<R> make_segsum(int key, int lane, R *dst) {
-   SegSum<R> sg;
-   sg.same = 0;
-#pragma unroll
-   for (int o = 0; o < 5; o++) {
-      const int k2 = __shfl_down_sync(kFull, key, 1 << o);
-      if (lane + (1 << o) < 32 && k2 == key) sg.same |= 1u << o;
-   }
-   const int kp = __shfl_up_sync(kFull, key, 1);
-   sg.head = key >= 0 && (lane == 0 || kp != key);
-   sg.dst = dst;
-   return sg;
-}
-
 // R = double: the FP64 path; R = float: the FP32 path (G_m series, VRR, image sum and the stored
 // targets in FP32; the geometry and every screening decision in FP64 as on the FP64 path).
 template <int LA, int LB, int LC, int LD, class R>
 __global__ void __launch_bounds__(Prim3Shape<LA, LB, LC, LD>::THREADS, Prim3Shape<LA, LB, LC, LD>::MINB)
-k_prim3(DevCtx ctx, BatchArgs bt) {
+k_prim3(DevCtx ctx, BatchArgs bt, int cp) {
    using Sh = Prim3Shape<LA, LB, LC, LD>;
    using G = typename Sh::G;
    constexpr int L = Sh::L, LF = Sh::LF, S = Sh::S, CP = Sh::CP;
@@ -96,35 +64,35 @@ k_prim3(DevCtx ctx, BatchArgs bt) {
    extern __shared__ __align__(16) double smem[];
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
    const int Ng = ctx.Ng;
-   // the image vectors, shared by the block
-   double *sneigh = smem;
-   for (int i = threadIdx.x; i < 3 * Ng; i += blockDim.x) sneigh[i] = __ldg(ctx.neighs + i);
+   // the image vectors in order of length, shared by the block
+   double4 *simg = reinterpret_cast<double4 *>(smem);
+   for (int i = threadIdx.x; i < 4 * Ng; i += blockDim.x) smem[i] = __ldg(reinterpret_cast<const double *>(ctx.img) + i);
    __syncthreads();
-   double *wbase = smem + ((3 * Ng + 1) & ~1) + (size_t)warp * Sh::WD;
+   double *wbase = smem + 4 * Ng + (size_t)warp * Sh::WD;
    PrimGeo *geo = reinterpret_cast<PrimGeo *>(wbase);
    R *acc = reinterpret_cast<R *>(wbase + CP * Sh::PG);
    double *q1t = wbase + CP * Sh::PG + CP * S;
    int *q1i = reinterpret_cast<int *>(q1t + 64);
    R *q2f = reinterpret_cast<R *>(q1t + 64 + 32);
    int *q2i = reinterpret_cast<int *>(q1t + 64 + 32 + 64 * LF);
-   // pair numbering within a chunk: pair = p * Ng + n3; each round of 32 pairs advances a lane
-   // by 32 = adv_p * Ng + adv_n
-   const int adv_p = 32 / Ng, adv_n = 32 - adv_p * Ng;
    const unsigned below = (1u << lane) - 1u;
    unsigned long long c_cheb = 0, c_boys = 0, c_vrr = 0;
 
-   const uint32_t nchunk = (bt.nprm + CP - 1) / CP;
+   const uint32_t nchunk = (bt.nprm + cp - 1) / cp;
    for (uint32_t ch = blockIdx.x * nwarp + warp; ch < nchunk; ch += gridDim.x * nwarp) {
-      const uint32_t p0 = ch * CP;
-      const int np = (int)min((uint32_t)CP, bt.nprm - p0);
+      const uint32_t p0 = ch * cp;
+      const int np = (int)min((uint32_t)cp, bt.nprm - p0);
+      int nimg = 0, start;
       if (lane < np) {
          PrimGeo g;
          const ShellRec sh = bt.shells[bt.prm_shell[p0 + lane]];
          prim_geometry(ctx, sh, bt.prm[p0 + lane], g);
          kill_if_screened(bt, sh, g);
          geo[lane] = g;
+         nimg = image_count(simg, Ng, g);
       }
-      for (int j = lane; j < CP * S; j += 32) acc[j] = R(0);
+      const int npair = pair_starts(nimg, np, lane, start);
+      for (int j = lane; j < np * S; j += 32) acc[j] = R(0);
       __syncwarp();
 
       int n1 = 0, n2 = 0;
@@ -135,9 +103,11 @@ k_prim3(DevCtx ctx, BatchArgs bt) {
          const int p = pk >> 8, n3 = pk & 255;
          const PrimGeo &g = geo[p];
          R z[17], F[LF];
+         const double4 im = simg[n3];
+         const double gv[3] = {im.x, im.y, im.z};
 #pragma unroll
          for (int q = 0; q < 3; q++) {
-            const double Qp = g.Q[q] + sneigh[n3 * 3 + q];
+            const double Qp = g.Q[q] + gv[q];
             const double W = wdist(g.zab, g.P[q], g.zcd, Qp, g.inv_z);
             z[q] = (R)g.PA[q];
             z[3 + q] = (R)(W - g.P[q]);
@@ -206,17 +176,18 @@ k_prim3(DevCtx ctx, BatchArgs bt) {
             }
          }
       };
-      // stage 2: truncation test over every (primitive, image) pair of the chunk
-      const int npair = np * Ng;
-      int tp = lane / Ng, tn = lane - (lane / Ng) * Ng;
+      // stage 2: truncation test over the (primitive, image) pairs of the chunk
       for (int b0 = 0; b0 < npair; b0 += 32) {
          bool pass = false;
          double T = 0.0;
+         int tn;
+         const int tp = pair_prim(b0, start, lane, tn);
          if (b0 + lane < npair) {
             const PrimGeo &g = geo[tp];
-            const double d0 = rsub(g.D[0], sneigh[tn * 3 + 0]);
-            const double d1 = rsub(g.D[1], sneigh[tn * 3 + 1]);
-            const double d2 = rsub(g.D[2], sneigh[tn * 3 + 2]);
+            const double4 im = simg[tn];
+            const double d0 = rsub(g.D[0], im.x);
+            const double d1 = rsub(g.D[1], im.y);
+            const double d2 = rsub(g.D[2], im.z);
             T = rmul(g.rho, rdot3(d0, d0, d1, d1, d2, d2));
             pass = !(T > g.upper);
          }
@@ -227,9 +198,6 @@ k_prim3(DevCtx ctx, BatchArgs bt) {
             q1t[pos] = T;
          }
          n1 += __popc(bal);
-         tp += adv_p;
-         tn += adv_n;
-         if (tn >= Ng) { tn -= Ng; tp++; }
          __syncwarp();
          if (n1 >= 32) {
             run_fm(32);
@@ -269,15 +237,22 @@ template <int LA, int LB, int LC, int LD, class R>
 cudaError_t launch_one(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st) {
    using Sh = Prim3Shape<LA, LB, LC, LD>;
    const size_t warp_bytes = (size_t)Sh::WD * 8;
-   const size_t neigh_bytes = (size_t)((3 * ctx.Ng + 1) & ~1) * 8;
+   const size_t neigh_bytes = (size_t)ctx.Ng * sizeof(double4);
    // shared memory per block sized so that MINB blocks share an SM
    const size_t budget = (220 * 1024) / Sh::MINB;
    const int maxw = Sh::THREADS / 32;
-   const int nw = (int)std::max<size_t>(1, std::min<size_t>(maxw, (budget - std::min(budget, neigh_bytes)) / warp_bytes));
+   const int nwmax = (int)std::max<size_t>(1, std::min<size_t>(maxw, (budget - std::min(budget, neigh_bytes)) / warp_bytes));
+   // A segment too small to give every resident warp CP primitives is cut finer, but not below what
+   // fills a G_m batch (one pair each without images, about four each with them), and it is spread
+   // over the SMs before a block takes more warps.
+   const long slots = 148L * Sh::MINB * nwmax;
+   const int cpmin = ctx.Ng == 1 ? Sh::CP : std::min(8, Sh::CP);
+   const int cp = (int)std::max((long)cpmin, std::min((long)Sh::CP, ((long)bt.nprm + slots - 1) / slots));
+   const long nchunk = ((long)bt.nprm + cp - 1) / cp;
+   const int nw = (int)std::max(1L, std::min((long)nwmax, (nchunk + 147) / 148));
    const size_t smem = neigh_bytes + warp_bytes * nw;
-   const long nchunk = ((long)bt.nprm + Sh::CP - 1) / Sh::CP;
    const long blocks = std::max(1L, std::min((nchunk + nw - 1) / nw, 148L * 24));
-   k_prim3<LA, LB, LC, LD, R><<<(unsigned)blocks, nw * 32, smem, st>>>(ctx, bt);
+   k_prim3<LA, LB, LC, LD, R><<<(unsigned)blocks, nw * 32, smem, st>>>(ctx, bt, cp);
    return cudaGetLastError();
 }
 

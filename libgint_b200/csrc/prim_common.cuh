@@ -46,10 +46,6 @@ static __device__ __forceinline__ void boys_eval_t(int nmax_rt, double T, double
    for (int n = 0; n <= nmax; n++) f[n] *= fac;
 }
 
-static __device__ void boys_eval(int nmax, double T, double *f, const double *__restrict__ ft, double fac) {
-   boys_eval_t<-1>(nmax, T, f, ft, fac);
-}
-
 // ---------------------------------------------------------------------------------------
 // Geometry that feeds discrete decisions. The minimum-image rounding (which lattice shift
 // brings Q next to P, and so which 27 images the image sum covers), the truncation test, the
@@ -170,17 +166,46 @@ static __device__ __forceinline__ void kill_if_screened(const BatchArgs &bt, con
    if (bt.gflags && !__ldg(bt.gflags + sh.group)) g.upper = -1.0;
 }
 
-// T = rho |P - Q - neighs[n3]|^2 (reference src/compute_Fm.cpp:204-210)
-static __device__ __forceinline__ double image_T(const DevCtx &ctx, const PrimGeo &g, int n3) {
-   const double PQ0 = rsub(g.D[0], __ldg(ctx.neighs + n3 * 3 + 0));
-   const double PQ1 = rsub(g.D[1], __ldg(ctx.neighs + n3 * 3 + 1));
-   const double PQ2 = rsub(g.D[2], __ldg(ctx.neighs + n3 * 3 + 2));
-   return rmul(g.rho, rdot3(PQ0, PQ0, PQ1, PQ1, PQ2, PQ2));
+// How many of the images, in order of their length, can pass the truncation test of a primitive:
+// rho |D - g|^2 <= upper needs |g| <= |D| + sqrt(upper / rho). The bound is widened by far more than
+// the test's rounding, so it leaves out only images that the test refuses; at least one is kept, so
+// that every primitive has a place in the pair numbering. (An undefined bound keeps all.) With 125
+// images of a 12.4 A cell and a 6 A range it keeps 7 to 20, of which 2 to 3 pass: on a 1/4096
+// sample of the 64-molecule l <= 3 workload the (ss|ss) primitive kernel went from 1.58 to 0.84 ms,
+// the classes of L <= 4 from 29.3 to 21.5 ms.
+static __device__ __forceinline__ int image_count(const double4 *img, int Ng, const PrimGeo &g) {
+   if (Ng == 1 || g.upper < 0.0) return 1;
+   const double rad = (sqrt(g.D[0] * g.D[0] + g.D[1] * g.D[1] + g.D[2] * g.D[2]) + sqrt(g.upper / g.rho)) * (1.0 + 1e-9);
+   int lo = 1, hi = Ng;
+   while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (img[mid - 1].w > rad) hi = mid - 1;
+      else lo = mid;
+   }
+   return lo;
 }
 
-// the truncation bound R^2 + 11 R + 50 (reference src/t_c_g0_n.cpp:78)
-static __device__ __forceinline__ double trunc_upper(double R) {
-   return radd(radd(rmul(R, R), rmul(11.0, R)), 50.0);
+// Numbers the (primitive, image) pairs of a chunk, primitive by primitive: lane p's primitive has n
+// pairs (n >= 1 for lane < np) from pair `start` on. Returns the pair count.
+static __device__ __forceinline__ int pair_starts(int n, int np, int lane, int &start) {
+   int sum = lane < np ? n : 0;
+#pragma unroll
+   for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= o) sum += u;
+   }
+   start = lane < np ? sum - n : 0x7fffffff;
+   return __shfl_sync(0xffffffffu, sum, 31);
+}
+
+// The primitive of pair b0 + lane, and its image's number among the primitive's.
+static __device__ __forceinline__ int pair_prim(int b0, int start, int lane, int &n3) {
+   const unsigned rel = (unsigned)start - (unsigned)b0;
+   const unsigned starts = __reduce_or_sync(0xffffffffu, start >= b0 && rel < 32u ? 1u << rel : 0u);
+   const int before = __popc(__ballot_sync(0xffffffffu, start < b0));
+   const int p = before + __popc(starts & ((2u << lane) - 1u)) - 1;
+   n3 = b0 + lane - __shfl_sync(0xffffffffu, start, p);
+   return p;
 }
 
 // four consecutive doubles from a 32-byte aligned, read-only global address
@@ -189,10 +214,10 @@ static __device__ __forceinline__ void ldg_v4(const double *p, double *v) {
 }
 
 // The degree-13 triangular Chebyshev series of one patch at (X1, X2), orders 0..L, times Kfac
-// (reference src/t_c_g0_n.cpp:133-178).
+// (reference src/t_c_g0_n.cpp:133-178); of them k0, k0 + kstep, ... only.
 template <int LT>
 static __device__ __forceinline__ void cheb_eval(const DevCtx &ctx, int L_rt, int patch, double X1, double X2,
-                                                 double Kfac, double *res) {
+                                                 double Kfac, double *res, int k0 = 0, int kstep = 1) {
    const int L = LT >= 0 ? LT : L_rt;
    const double B1 = __ldg(ctx.bw + patch * 4 + 0), W1 = __ldg(ctx.bw + patch * 4 + 1);
    const double B2 = __ldg(ctx.bw + patch * 4 + 2), W2 = __ldg(ctx.bw + patch * 4 + 3);
@@ -209,7 +234,7 @@ static __device__ __forceinline__ void cheb_eval(const DevCtx &ctx, int L_rt, in
       T1[i] = 2. * TG1 * T1[i - 1] - T1[i - 2];
       T2[i] = 2. * TG2 * T2[i - 1] - T2[i - 2];
    }
-   for (int k = 0; k <= L; k++) {
+   for (int k = k0; k <= L; k += kstep) {
       // one 32-byte load per four coefficients (each lane reads its own patch, so a narrower
       // load would fetch every sector four times)
       const double *c = C0_row + k * kC0Row;
@@ -275,59 +300,19 @@ static __device__ __forceinline__ void cheb_eval_f(const DevCtx &ctx, int L_rt, 
 }
 
 // ---------------------------------------------------------------------------------------
-// Truncated-Coulomb G_m(T,R) * Kfac (reference src/t_c_g0_n.cpp:67-180); falls back to the
-// Boys function for R > 11 and T < R^2 - 11 R.
+// Truncated-Coulomb G_m(T,R) * Kfac (reference src/t_c_g0_n.cpp:67-180); the Boys function for
+// R > 11 and T < R^2 - 11 R. LT >= 0 fixes L at compile time (the loops unroll); LT < 0 takes L_rt.
 // ---------------------------------------------------------------------------------------
-// returns 0 when T is beyond the truncation (zeros), 1 for the Chebyshev series, 2 for Boys
-// LT >= 0 fixes L at compile time (the loops unroll); LT < 0 takes L_rt.
-template <int LT>
-static __device__ __forceinline__ int fm_eval_t(const DevCtx &ctx, int L_rt, double R, double T, double Kfac,
-                                                double *res) {
-   const int L = LT >= 0 ? LT : L_rt;
-   double upper = trunc_upper(R);
-   double lower = radd(rsub(rmul(R, R), rmul(11.0, R)), 0.0);
-   double X1, X2;
-   int patch;
-   if (T > upper) {
-      for (int n = 0; n <= L; n++) res[n] = 0.0;
-      return 0;
-   }
-   if (R <= 11.0) {
-      X2 = R / 11.0;
-      lower = 0.0;
-      X1 = rsub(T, lower) / rsub(upper, lower);
-      int i1 = (int)(X1 * 128), i2 = (int)(X2 * 128);
-      if (i1 == 128) i1 = 127;
-      if (i2 == 128) i2 = 127;
-      patch = __ldg(ctx.lut_low + i1 * 128 + i2);
-   } else {
-      if (T < lower) {
-         boys_eval_t<LT>(L, T, res, ctx.ftable, Kfac);
-         return 2;
-      }
-      X2 = 11.0 / R;
-      X1 = rsub(T, lower) / rsub(upper, lower);
-      int i1 = (int)(X1 * 128), i2 = (int)(X2 * 128);
-      if (i1 == 128) i1 = 127;
-      if (i2 == 128) i2 = 127;
-      patch = __ldg(ctx.lut_high + i1 * 128 + i2);
-   }
-   cheb_eval<LT>(ctx, L, patch, X1, X2, Kfac, res);
-   return 1;
-}
-
-static __device__ int fm_eval(const DevCtx &ctx, int L, double R, double T, double Kfac, double *res) {
-   return fm_eval_t<-1>(ctx, L, R, T, Kfac, res);
-}
-
-// G_m * Kfac of one image from the primitive's precomputed bounds and X2; the same decisions and
-// arithmetic as fm_eval_t. Returns 0 beyond the truncation, 1 for the series, 2 for Boys.
+// G_m * Kfac of one image from the primitive's precomputed bounds and X2, with the reference's
+// decisions. Returns 0 beyond the truncation, 1 for the series, 2 for Boys. k0 and kstep: of the
+// series' orders only k0, k0 + kstep, ... (several threads share one image; Boys gives all of them
+// to k0 = 0).
 template <int LT>
 static __device__ __forceinline__ int fm_eval_geo(const DevCtx &ctx, int L_rt, const PrimGeo &g, double T,
-                                                  double *res) {
+                                                  double *res, int k0 = 0, int kstep = 1) {
    const int L = LT >= 0 ? LT : L_rt;
    if (T > g.upper) {
-      for (int n = 0; n <= L; n++) res[n] = 0.0;
+      for (int n = k0; n <= L; n += kstep) res[n] = 0.0;
       return 0;
    }
    double X1;
@@ -339,7 +324,7 @@ static __device__ __forceinline__ int fm_eval_geo(const DevCtx &ctx, int L_rt, c
       patch = __ldg(ctx.lut_low + i1 * 128 + g.i2);
    } else {
       if (T < g.lower) {
-         boys_eval_t<LT>(L, T, res, ctx.ftable, g.Kfac);
+         if (k0 == 0) boys_eval_t<LT>(L, T, res, ctx.ftable, g.Kfac);
          return 2;
       }
       X1 = rsub(T, g.lower) / rsub(g.upper, g.lower);
@@ -347,7 +332,7 @@ static __device__ __forceinline__ int fm_eval_geo(const DevCtx &ctx, int L_rt, c
       if (i1 == 128) i1 = 127;
       patch = __ldg(ctx.lut_high + i1 * 128 + g.i2);
    }
-   cheb_eval<LT>(ctx, L, patch, X1, g.X2, g.Kfac, res);
+   cheb_eval<LT>(ctx, L, patch, X1, g.X2, g.Kfac, res, k0, kstep);
    return 1;
 }
 
@@ -375,6 +360,38 @@ static __device__ __forceinline__ uint32_t row_group_one(const BatchArgs &bt, ui
    const uint32_t gi = g0 + 1u + (uint32_t)lane;
    const bool later = gi < bt.ngroup && __ldg(&bt.groups[gi].qrtt_off) <= q;
    return g0 + __popc(__ballot_sync(0xffffffffu, later));
+}
+
+// Segmented sum over adjacent lanes that carry the same key (keys are contiguous runs); the
+// first lane of each run adds the run's sum to dst[s]. R = double, or float on the FP32 path.
+template <class R>
+struct SegSum {
+   unsigned same;   // bit o: lane + 2^o carries this lane's key
+   bool head;
+   R *dst;
+   __device__ __forceinline__ void operator()(int s, R v) {
+#pragma unroll
+      for (int o = 0; o < 5; o++) {
+         const R u = __shfl_down_sync(0xffffffffu, v, 1 << o);
+         if (same & (1u << o)) v += u;
+      }
+      if (head) dst[s] += v;
+   }
+};
+
+template <class R>
+static __device__ __forceinline__ SegSum<R> make_segsum(int key, int lane, R *dst) {
+   SegSum<R> sg;
+   sg.same = 0;
+#pragma unroll
+   for (int o = 0; o < 5; o++) {
+      const int k2 = __shfl_down_sync(0xffffffffu, key, 1 << o);
+      if (lane + (1 << o) < 32 && k2 == key) sg.same |= 1u << o;
+   }
+   const int kp = __shfl_up_sync(0xffffffffu, key, 1);
+   sg.head = key >= 0 && (lane == 0 || kp != key);
+   sg.dst = dst;
+   return sg;
 }
 
 // fm_eval_geo for the FP32 path: the same decisions (truncation, branch, patch) in FP64, the
