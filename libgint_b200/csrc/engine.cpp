@@ -551,14 +551,18 @@ static cudaStream_t worker_for(Handle *h, int i, bool uses_scratch) {
    return uses_scratch ? h->work[0] : h->work[1 + i % (kWorkStreams - 1)];
 }
 
+// Doubles from a segment's image-summed targets to its shell quartets' displacements (BatchArgs::sgeo).
+static size_t sgeo_offset(Handle *h, int c, size_t nprm) { return (nprm * h->plans[c & 255].S + 3) & ~(size_t)3; }
+
 // The worker stream (index) that a replay gives its i-th recorded segment (of class c), as
-// worker_for does, and the image-summed targets that segment needs (doubles, 32-byte multiple).
+// worker_for does, and the image-summed targets and displacements that segment needs (doubles,
+// 32-byte multiple).
 static int replay_worker(Handle *h, int c, int i) {
    int a, b;
    return group_global_scratch(h->plans[c & 255], &a, &b) != 0 ? 0 : 1 + i % (kWorkStreams - 1);
 }
-static size_t replay_seg_ac(Handle *h, int c, uint32_t nprm) {
-   return ((size_t)nprm * h->plans[c & 255].S + 3) & ~(size_t)3;
+static size_t replay_seg_ac(Handle *h, int c, uint32_t nprm, uint32_t nshell) {
+   return sgeo_offset(h, c, nprm) + (((size_t)6 * nshell + 3) & ~(size_t)3);
 }
 
 static DevCtx make_ctx(Handle *h) {
@@ -654,7 +658,7 @@ static void flush(Handle *h) {
       g.o_q = off; off = al16(off + Q.qrtts.size() * sizeof(QrttRec));
       g.o_rg = off; off = al16(off + Q.rowgrp.size() * 4);
       g.ac_off = ac;
-      ac += ((size_t)Q.prm.size() * h->plans[c & 255].S + 1) & ~(size_t)1;
+      ac += replay_seg_ac(h, c, (uint32_t)Q.prm.size(), (uint32_t)Q.shells.size());
       segs.push_back(g);
    }
    if (!ensure(h, s.rec, std::max(off, (size_t)(64u << 20)), "record buffer")) return;
@@ -707,6 +711,7 @@ static void flush(Handle *h) {
       bt.ngroup = (uint32_t)Q.groups.size();
       bt.nqrtt = (uint32_t)Q.qrtts.size();
       bt.AC = (double *)s.ac.p + g.ac_off;
+      bt.sgeo = bt.AC + sgeo_offset(h, g.c, bt.nprm);
       int gg = 0, gw = 0;
       size_t gs = group_global_scratch(hp, &gg, &gw);
       if (gs) {
@@ -882,6 +887,7 @@ static bool enqueue_replay(Handle *h, const DevCtx &ctx, std::vector<cudaEvent_t
          // one after another, and no other stream touches that arena
          const int w = replay_worker(h, g.c, nseg++);
          bt.AC = (double *)h->rec_ac.p + h->arena_off[w];
+         bt.sgeo = bt.AC + sgeo_offset(h, g.c, g.nprm);
          bt.gscratch = (double *)h->rec_gscr.p;
          const ClassPlan &hp = h->plans[g.c & 255];
          cudaStream_t st = spread ? h->work[w] : h->stream;
@@ -932,7 +938,7 @@ static bool prepare_replay(Handle *h, size_t *half) {
    for (auto &rb : h->recs)
       for (auto &g : rb.segs) {
          const int w = replay_worker(h, g.c, i++);
-         arena[w] = std::max(arena[w], replay_seg_ac(h, g.c, g.nprm));
+         arena[w] = std::max(arena[w], replay_seg_ac(h, g.c, g.nprm, g.nshell));
          int a, b;
          gs = std::max(gs, group_global_scratch(h->plans[g.c & 255], &a, &b));
       }
@@ -1155,10 +1161,11 @@ static int autotune_impl(Handle *h, int *out) {
          bt.rowgrp = (const uint32_t *)(base + g.o_rg);
          bt.nprm = g.nprm; bt.nshell = g.nshell; bt.ngroup = g.ngroup; bt.nqrtt = g.nqrtt;
          bt.AC = (double *)h->rec_ac.p + h->arena_off[wk];
+         bt.sgeo = bt.AC + sgeo_offset(h, g.c, g.nprm);
          bt.gscratch = (double *)h->rec_gscr.p;
          seen[c] = true;
          alt_p[c] = prim_has_generated(c);
-         alt_g[c] = true;   // variant 0: k_group3, or k_group_block where it applies; variant 1: k_group
+         alt_g[c] = true;   // variant 0: k_group3 or k_group_mm; variant 1: k_group
          ck(h, cudaEventRecord(ev[0], h->stream), "event");
          bt.prim_variant = 1;
          ck(h, launch_prim(ctx, bt, hp, h->stream), "k_prim launch");
@@ -1222,7 +1229,11 @@ void libgint_init(void *hh) {
    static std::once_flag loaded[kMaxDevices];
    if (h->device >= 0 && h->device < kMaxDevices) {
       cudaError_t pe = cudaSuccess;
-      std::call_once(loaded[h->device], [&]() { pe = preload_kernels(); });
+      std::call_once(loaded[h->device], [&]() {
+         double c2s[4][70];
+         make_c2s(c2s);
+         pe = preload_kernels(&c2s[0][0]);
+      });
       ck(h, pe, "kernel preload");
       if (!h->err && !group_prog(h->device)) set_error(h, 4, "kernel preload: no HRR instructions on this device");
    }
@@ -1542,7 +1553,7 @@ static void commit_group(Handle *h, ClassQ &Q, int qcls, uint32_t shell0, uint32
    }
    if (!Q.active) { Q.active = true; h->active.push_back(qcls); }
    h->pend_prims += nprm;
-   h->pend_ac += nprm * S;
+   h->pend_ac += nprm * S + 6 * (Q.shells.size() - shell0);
    h->pend_rec += recs;
 }
 
@@ -1858,7 +1869,11 @@ int libgint_replay_noalloc(void *hh, const double *P_dev, double *K_dev, size_t 
          bt.rowgrp = (const uint32_t *)(base + g.o_rg);
          bt.nprm = g.nprm; bt.nshell = g.nshell; bt.ngroup = g.ngroup; bt.nqrtt = g.nqrtt;
          bt.AC = scr;                                                   // segments run in stream order
-         bt.gscratch = scr + (((size_t)g.nprm * hp.S + 31) & ~(size_t)31);
+         const size_t gs0 = ((size_t)g.nprm * hp.S + 31) & ~(size_t)31;
+         bt.gscratch = scr + gs0;
+         int ga = 0, gb = 0;
+         const size_t sg0 = gs0 + ((group_global_scratch(hp, &ga, &gb) + 3) & ~(size_t)3);
+         if (sg0 + (size_t)6 * g.nshell <= kNoAllocScratchDoubles) bt.sgeo = scr + sg0;   // else derived by their readers
          if (!ck(h, launch_prim(ctx, bt, hp, st), "libgint_replay_noalloc: k_prim launch")) return h->err;
          if (!ck(h, launch_group(ctx, bt, hp, st), "libgint_replay_noalloc: k_group launch")) return h->err;
       }

@@ -32,6 +32,84 @@ __device__ __forceinline__ double symm_factor(int i) {
    return i == 0 ? 2.0 : (i == 1 ? 1.0 : (i == 2 ? 0.5 : (i == 3 ? 0.25 : 0.0)));
 }
 
+// One spin's K update of one row from its spherical block I (reference src/compute_KS.cpp:26-115):
+// K_bd -= f I P_ac and its three partners, each summed over the block in registers first. A row of
+// (pp|ps) then reads 24 elements of P and adds 24 to K, where one read and one atomic per integral and
+// partner were 108 of each (classes of L <= 3 of the 1/4096 sample of the 64-molecule l <= 3 workload,
+// with the displacements read instead of derived: 14.1 to 12.9 ms).
+template <int NA, int NB, int NC, int ND, class R>
+static __device__ __forceinline__ void k_update(const R *I, const double *__restrict__ P, double *K, const QrttRec &k,
+                                                double f) {
+   // the element (x, y) of pair u (ac, ad, bc, bd) is at off[u] + x sx[u] + y sy[u]
+   int sx[4], sy[4];
+#pragma unroll
+   for (int u = 0; u < 4; u++) {
+      const bool T = (k.T >> u) & 1;
+      sx[u] = T ? (int)k.ld[u] : 1;
+      sy[u] = T ? 1 : (int)k.ld[u];
+   }
+   // all of P first: one round of independent loads
+   double Pac[NA][NC], Pad[NA][ND], Pbc[NB][NC], Pbd[NB][ND];
+#pragma unroll
+   for (int a = 0; a < NA; a++) {
+#pragma unroll
+      for (int c = 0; c < NC; c++) Pac[a][c] = __ldg(P + ((size_t)k.off[0] + a * sx[0] + c * sy[0]));
+#pragma unroll
+      for (int d = 0; d < ND; d++) Pad[a][d] = __ldg(P + ((size_t)k.off[1] + a * sx[1] + d * sy[1]));
+   }
+#pragma unroll
+   for (int b = 0; b < NB; b++) {
+#pragma unroll
+      for (int c = 0; c < NC; c++) Pbc[b][c] = __ldg(P + ((size_t)k.off[2] + b * sx[2] + c * sy[2]));
+#pragma unroll
+      for (int d = 0; d < ND; d++) Pbd[b][d] = __ldg(P + ((size_t)k.off[3] + b * sx[3] + d * sy[3]));
+   }
+#define I4(a, b, c, d) ((double)I[(((a) * NB + (b)) * NC + (c)) * ND + (d)])
+#pragma unroll
+   for (int b = 0; b < NB; b++) {
+#pragma unroll
+      for (int d = 0; d < ND; d++) {
+         double v = 0.0;
+#pragma unroll
+         for (int a = 0; a < NA; a++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) v += I4(a, b, c, d) * Pac[a][c];
+         atomicAdd(K + ((size_t)k.off[3] + b * sx[3] + d * sy[3]), f * v);
+      }
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+         double v = 0.0;
+#pragma unroll
+         for (int a = 0; a < NA; a++)
+#pragma unroll
+            for (int d = 0; d < ND; d++) v += I4(a, b, c, d) * Pad[a][d];
+         atomicAdd(K + ((size_t)k.off[2] + b * sx[2] + c * sy[2]), f * v);
+      }
+   }
+#pragma unroll
+   for (int a = 0; a < NA; a++) {
+#pragma unroll
+      for (int d = 0; d < ND; d++) {
+         double v = 0.0;
+#pragma unroll
+         for (int b = 0; b < NB; b++)
+#pragma unroll
+            for (int c = 0; c < NC; c++) v += I4(a, b, c, d) * Pbc[b][c];
+         atomicAdd(K + ((size_t)k.off[1] + a * sx[1] + d * sy[1]), f * v);
+      }
+#pragma unroll
+      for (int c = 0; c < NC; c++) {
+         double v = 0.0;
+#pragma unroll
+         for (int b = 0; b < NB; b++)
+#pragma unroll
+            for (int d = 0; d < ND; d++) v += I4(a, b, c, d) * Pbd[b][d];
+         atomicAdd(K + ((size_t)k.off[0] + a * sx[0] + c * sy[0]), f * v);
+      }
+   }
+#undef I4
+}
+
 // resident 128-thread blocks per SM the register budget is sized for: the kernel waits on
 // chains of dependent loads, so small classes trade registers for more warps in flight
 template <int LA, int LB, int LC, int LD>
@@ -46,8 +124,6 @@ template <int LA, int LB, int LC, int LD, class R>
 __global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB) k_group3(DevCtx ctx, BatchArgs bt) {
    using G = GrpGen<LA, LB, LC, LD>;
    constexpr int S = G::S, Nc = G::Nc, Ns = G::Ns;
-   constexpr int nsb = 2 * LB + 1, nsc = 2 * LC + 1, nsd = 2 * LD + 1;
-   constexpr int nscd = nsc * nsd, nsbcd = nsb * nscd;
    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
    const uint32_t nblk = (bt.nqrtt + 31) >> 5;
    // one lane per contraction row: a warp takes 32 consecutive rows, so the lanes of one set
@@ -65,8 +141,8 @@ __global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB) k_grou
       for (int t = 0; t < Nc; t++) cart[t] = R(0);
       for (uint32_t s = 0; s < Gr.nshell; s++) {
          const ShellRec sh = bt.shells[Gr.shell_off + s];
-         const BasisEnt ea = ctx.ents[sh.ent[0]], eb = ctx.ents[sh.ent[1]];
-         const BasisEnt ec = ctx.ents[sh.ent[2]], ed = ctx.ents[sh.ent[3]];
+         const BasisEnt &ea = ctx.ents[sh.ent[0]], &eb = ctx.ents[sh.ent[1]];
+         const BasisEnt &ec = ctx.ents[sh.ent[2]], &ed = ctx.ents[sh.ent[3]];
          const double *Ka = ctx.pool + ea.k_off + ia * ea.np;
          const double *Kb = ctx.pool + eb.k_off + ib * eb.np;
          const double *Kc = ctx.pool + ec.k_off + ic * ec.np;
@@ -86,39 +162,21 @@ __global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB) k_grou
 #pragma unroll
             for (int j = 0; j < S; j++) T[j] += kp * __ldg(row + j);
          }
-         double A[3], B[3], C[3], D[3], CDs[3];
-         shell_geom(ctx, ea, eb, ec, ed, sh.n1, sh.n2, A, B, C, D, CDs);
-         const R AB[3] = {(R)(A[0] - B[0]), (R)(A[1] - B[1]), (R)(A[2] - B[2])};
-         const R CD[3] = {(R)(C[0] - D[0]), (R)(C[1] - D[1]), (R)(C[2] - D[2])};
+         double v[6];
+         read_shell_vectors(ctx, bt, Gr.shell_off + s, sh, v);
+         const R AB[3] = {(R)v[0], (R)v[1], (R)v[2]}, CD[3] = {(R)v[3], (R)v[4], (R)v[5]};
          G::hrr(T, AB, CD, cart);
       }
       R sph[Ns];
       G::sph(cart, sph);
       const QrttRec k = bt.qrtts[q];
       const double fac = symm_factor(k.idx_fac) * ctx.hf_fac;
-#pragma unroll
-      for (int t = 0; t < Ns; t++) {
-         const int isa = t / nsbcd, isb = (t / nscd) % nsb, isc = (t / nsd) % nsc, isd = t % nsd;
-         const int iac = !(k.T & 1) ? isc * k.ld[0] + isa : isa * k.ld[0] + isc;
-         const int iad = !(k.T & 2) ? isd * k.ld[1] + isa : isa * k.ld[1] + isd;
-         const int ibc = !(k.T & 4) ? isc * k.ld[2] + isb : isb * k.ld[2] + isc;
-         const int ibd = !(k.T & 8) ? isd * k.ld[3] + isb : isb * k.ld[3] + isd;
-         const size_t Iac = (size_t)k.off[0] + iac, Iad = (size_t)k.off[1] + iad;
-         const size_t Ibc = (size_t)k.off[2] + ibc, Ibd = (size_t)k.off[3] + ibd;
-         if (Iac >= ctx.FP_size || Iad >= ctx.FP_size || Ibc >= ctx.FP_size || Ibd >= ctx.FP_size) {
-            atomicOr(ctx.err, 1);
-            continue;
-         }
-         const double iabcd = -fac * (double)sph[t];
-         for (int sp = 0; sp < ctx.nspin; sp++) {
-            const double *Pm = ctx.P[sp];
-            double *Km = ctx.K[sp];
-            atomicAdd(Km + Ibd, iabcd * __ldg(Pm + Iac));
-            atomicAdd(Km + Ibc, iabcd * __ldg(Pm + Iad));
-            atomicAdd(Km + Iad, iabcd * __ldg(Pm + Ibc));
-            atomicAdd(Km + Iac, iabcd * __ldg(Pm + Ibd));
-         }
+      if (!row_in_range(k, 2 * LA + 1, 2 * LB + 1, 2 * LC + 1, 2 * LD + 1, ctx.FP_size)) {
+         atomicOr(ctx.err, 1);
+         continue;
       }
+      for (int sp = 0; sp < ctx.nspin; sp++)
+         k_update<2 * LA + 1, 2 * LB + 1, 2 * LC + 1, 2 * LD + 1>(sph, ctx.P[sp], ctx.K[sp], k, -fac);
    }
 }
 

@@ -9,10 +9,11 @@
 //               surviving image, generated per lane (prim3.cu) or interpreted by a team (below).
 //               (reference: src/compute_Fm.cpp:20-326, src/compute_VRR.cpp:349-458,
 //                src/compute_ECO.cpp:216-272)
-//  k_group      one warp per group (all image pairs of one set quartet for one class): for
-//               every contraction row, contract AC over the primitives of each shell, apply
-//               the HRR with that shell's AB/CD, sum the shells, transform to spherical and
-//               update K with atomics.
+//  k_group3, k_group_mm, k_group   for every contraction row of every group (all image pairs of one set
+//               quartet), contract AC over the primitives of each shell, apply the HRR with that
+//               shell's AB/CD, sum the shells, transform to spherical and update K with atomics:
+//               one lane per row (group3.cu), one block per group (group_mm.cuh), or one warp per
+//               row (below).
 //               (reference: src/compute_ECO.cpp:12-214, src/compute_HRR.cpp:102-225,
 //                src/compute_SPH.cpp:58-237, src/compute_KS.cpp:8-117)
 #include <cuda_runtime.h>
@@ -23,6 +24,7 @@
 #include "engine_types.h"
 #include "kernels.h"
 #include "group3.h"
+#include "group_mm.h"
 #include "prim3.h"
 #include "prim_common.cuh"
 
@@ -64,6 +66,7 @@ template <int NT>
 __global__ void __launch_bounds__(NT == 32 ? 256 : NT, NT == 32 ? 2 : (NT == 128 ? 4 : 1))
 k_prim2(DevCtx ctx, BatchArgs bt, int cp, int team_doubles) {
    extern __shared__ __align__(16) double smem[];
+   write_shell_vectors(ctx, bt);
    ClassPlan *pl = reinterpret_cast<ClassPlan *>(smem);
    {
       const int nwords = (int)(sizeof(ClassPlan) / 4);
@@ -293,15 +296,16 @@ struct ShellShared {
 };
 static_assert(sizeof(ShellShared) <= kGroupShellCacheDoubles * 8, "shell cache slot too small");
 
-static __device__ __forceinline__ void shell_shared(const DevCtx &ctx, const ShellRec &sh, ShellShared &o) {
-   const BasisEnt ea = ctx.ents[sh.ent[0]], eb = ctx.ents[sh.ent[1]];
-   const BasisEnt ec = ctx.ents[sh.ent[2]], ed = ctx.ents[sh.ent[3]];
+static __device__ __forceinline__ void shell_shared(const DevCtx &ctx, const BatchArgs &bt, uint32_t i, ShellShared &o) {
+   const ShellRec sh = bt.shells[i];
    o.prm_off = sh.prm_off; o.nprm = sh.nprm;
-   o.k_off[0] = ea.k_off; o.k_off[1] = eb.k_off; o.k_off[2] = ec.k_off; o.k_off[3] = ed.k_off;
-   o.np[0] = ea.np; o.np[1] = eb.np; o.np[2] = ec.np; o.np[3] = ed.np;
-   double A[3], B[3], C[3], D[3], CDs[3];
-   shell_geom(ctx, ea, eb, ec, ed, sh.n1, sh.n2, A, B, C, D, CDs);
-   for (int c = 0; c < 3; c++) { o.AB[c] = A[c] - B[c]; o.CD[c] = C[c] - D[c]; }
+   for (int q = 0; q < 4; q++) {
+      const BasisEnt &e = ctx.ents[sh.ent[q]];
+      o.k_off[q] = e.k_off; o.np[q] = e.np;
+   }
+   double v[6];
+   read_shell_vectors(ctx, bt, i, sh, v);
+   for (int c = 0; c < 3; c++) { o.AB[c] = v[c]; o.CD[c] = v[3 + c]; }
 }
 
 // One contraction row q (of group gi = G) processed by NL cooperating threads (a block, a warp or
@@ -327,7 +331,7 @@ static __device__ __forceinline__ void group_body(const DevCtx &ctx, const Batch
          if (cache && s == 0 && cache->key == gi) {
             sh = *cache;
          } else {
-            shell_shared(ctx, bt.shells[G.shell_off + s], sh);
+            shell_shared(ctx, bt, G.shell_off + s, sh);
             if (cache && s == 0) {
                gsync<NL>();
                if (lane == 0) { *cache = sh; cache->key = gi; }
@@ -512,53 +516,6 @@ __global__ void __launch_bounds__(256, 4) k_group(DevCtx ctx, BatchArgs bt, int 
    }
 }
 
-// one block of NT threads per contraction row, all of them on one workspace (in shared memory, or
-// for the largest classes a slice of the global scratch per block): for the classes whose rows are
-// long chains of HRR levels with hundreds to thousands of elements each and which have few rows,
-// a warp per row leaves the GPU mostly idle and takes a level in many rounds. NT = 128 (eight
-// blocks per SM at 64 registers) up to kGroupBlockWideDoubles of workspace, 256 above.
-template <int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT) k_group_block(DevCtx ctx, BatchArgs bt, int ws_doubles,
-                                                                int use_global) {
-   extern __shared__ __align__(16) double smem[];
-   const ClassPlan *pl = reinterpret_cast<const ClassPlan *>(smem);
-   load_plan(bt.plan, smem);
-   __syncthreads();
-   const int plan_doubles = (int)((sizeof(ClassPlan) + 15) / 16) * 2;
-   double *kpw = smem + plan_doubles;
-   double *ws = use_global ? bt.gscratch + (size_t)blockIdx.x * ws_doubles : kpw + kGroupKpDoubles;
-   const int Hws = max(pl->H, 2 * pl->Nc);
-   const uint2 *hrec = ctx.gprog + ctx.gprog[bt.cls].x;
-   const int lane = threadIdx.x & 31;
-   for (uint32_t q = blockIdx.x; q < bt.nqrtt; q += gridDim.x) {
-      const uint32_t gi = row_group_one(bt, q, lane);   // the same in every warp of the block
-      if (bt.gflags && !__ldg(bt.gflags + gi)) continue;   // screened on an incremental replay
-      const GroupRec G = bt.groups[gi];
-      group_body<NT, 1>(ctx, bt, pl, G, q, ws, ws + Hws, (int)threadIdx.x, hrec, kpw);
-   }
-}
-
-// one lane per contraction row, for classes with a small workspace (lane-interleaved in shared memory)
-__global__ void __launch_bounds__(256) k_group_lane(DevCtx ctx, BatchArgs bt, int lane_doubles) {
-   extern __shared__ __align__(16) double smem[];
-   const ClassPlan *pl = reinterpret_cast<const ClassPlan *>(smem);
-   load_plan(bt.plan, smem);
-   __syncthreads();
-   const int plan_doubles = (int)((sizeof(ClassPlan) + 15) / 16) * 2;
-   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nwarp = blockDim.x / 32;
-   double *wbase = smem + plan_doubles + (size_t)warp * 32 * lane_doubles + lane;
-   const int Hws = max(pl->H, 2 * pl->Nc);
-   const uint2 *hrec = ctx.gprog + ctx.gprog[bt.cls].x;
-   const uint32_t nblk = (bt.nqrtt + 31) >> 5;
-   for (uint32_t blk = blockIdx.x * nwarp + warp; blk < nblk; blk += gridDim.x * nwarp) {
-      const uint32_t q0 = blk << 5, q = q0 + lane;
-      const uint32_t gi = row_group_warp(bt, q0, lane);
-      if (q >= bt.nqrtt || (bt.gflags && !__ldg(bt.gflags + gi))) continue;
-      const GroupRec G = bt.groups[gi];
-      group_body<1, 32>(ctx, bt, pl, G, q, wbase, wbase + Hws * 32, 0, hrec, nullptr);
-   }
-}
-
 // ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
@@ -740,10 +697,9 @@ size_t group_global_scratch(const ClassPlan &hp, int *grid, int *warps) {
 }
 
 
-// Group-kernel choice: k_group3 (generated HRR, one lane per row) for the classes it covers; for
-// the others on variant 0 k_group_block (one block per row) where the workspace is large and fits
-// a block's shared memory, k_group_lane for small workspaces, else k_group (one warp per row),
-// which variant 1 always takes.
+// Group-kernel choice on variant 0: k_group3 (generated HRR, one lane per row) for the classes it
+// covers, k_group_mm (dense products, one block per group) for the others; on variant 1 always
+// k_group (one warp per row).
 cudaError_t launch_group(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan &hp, cudaStream_t st) {
    if (bt.nqrtt == 0) return cudaSuccess;
    if (bt.group_variant == 0 || bt.fp32) {
@@ -751,39 +707,8 @@ cudaError_t launch_group(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan
       if (group3_launch(ctx, bt, st, &err)) return err;
    }
    if (bt.fp32) return cudaErrorInvalidValue;   // FP32 segments exist only for classes with k_group3
+   if (bt.group_variant == 0) return group_mm_launch(ctx, bt, hp, max_dyn_smem(), st);
    const size_t wd = group_warp_doubles(hp);
-   if (bt.group_variant == 0 && wd >= (size_t)kGroupBlockMinDoubles) {
-      const bool wide = wd >= (size_t)kGroupBlockWideDoubles;
-      const size_t smem = group_hdr_bytes() + (kGroupKpDoubles + wd) * 8;
-      long blocks = 0;
-      int use_global = 0;
-      size_t dyn = smem;
-      if (smem <= (size_t)std::min(max_dyn_smem(), 200 * 1024)) {
-         blocks = std::max(1L, std::min((long)bt.nqrtt, 148L * 16));
-      } else if (bt.gscratch) {   // workspace in the global scratch, which holds group_global_scratch's count
-         int grid = 0, warps = 0;
-         group_global_scratch(hp, &grid, &warps);
-         blocks = std::max(1L, std::min((long)bt.nqrtt, (long)grid * warps));
-         use_global = 1;
-         dyn = group_hdr_bytes() + kGroupKpDoubles * 8;
-      }
-      if (blocks) {
-         if (wide) k_group_block<256><<<(unsigned)blocks, 256, dyn, st>>>(ctx, bt, (int)wd, use_global);
-         else k_group_block<128><<<(unsigned)blocks, 128, dyn, st>>>(ctx, bt, (int)wd, use_global);
-         return cudaGetLastError();
-      }
-   }
-   if (wd <= 40 && bt.group_variant == 0) {
-      // small workspace: one lane per group, 32 groups per warp
-      const int lane_doubles = (int)wd;
-      const size_t plan_bytes = group_hdr_bytes();
-      const int nw = 8;
-      const size_t smem = plan_bytes + (size_t)nw * 32 * lane_doubles * 8;
-      long blocks = ((long)bt.nqrtt + nw * 32 - 1) / (nw * 32);
-      blocks = std::max(1L, std::min(blocks, 148L * 16));
-      k_group_lane<<<(unsigned)blocks, nw * 32, smem, st>>>(ctx, bt, lane_doubles);
-      return cudaGetLastError();
-   }
    const size_t plan_bytes = group_hdr_bytes();
    const int nw = group_smem_warps(wd);
    if (nw >= 1) {
@@ -1003,12 +928,11 @@ const uint2 *group_prog(int device) {
 // kernel: set per launch (with the launch's own size), one caller thread could lower it between
 // another thread's setting and launch, which failed that launch ("invalid argument"). It is
 // therefore raised once, here, before any handle launches; launches pass only their own size.
-cudaError_t preload_kernels() {
+cudaError_t preload_kernels(const double *c2s_l0to3) {
    cudaError_t e;
    const int smax = max_dyn_smem();
    const void *fns[] = {(const void *)k_prim2<32>, (const void *)k_prim2<128>, (const void *)k_prim2<256>,
-                        (const void *)k_group, (const void *)k_group_lane, (const void *)k_group_block<128>,
-                        (const void *)k_group_block<256>};
+                        (const void *)k_group};
    for (const void *f : fns)
       if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smax)) != cudaSuccess) return e;
    cudaFuncAttributes a;
@@ -1017,6 +941,7 @@ cudaError_t preload_kernels() {
    if ((e = cudaFuncGetAttributes(&a, (const void *)k_row_groups)) != cudaSuccess) return e;
    if ((e = prim3_preload(smax)) != cudaSuccess) return e;
    if ((e = group3_preload()) != cudaSuccess) return e;
+   if ((e = group_mm_preload(smax, c2s_l0to3)) != cudaSuccess) return e;
    return group_prog_load();
 }
 

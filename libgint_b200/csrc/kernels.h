@@ -61,10 +61,11 @@ struct BatchArgs {
    const uint8_t *gflags;     // incremental replay: 0 = skip the group (its primitives and rows); null = all run
    double *AC;                // [nprm][S] image-summed VRR targets (floats in the first half for fp32)
    int fp32;                  // 1: the segment's shell quartets run in FP32 (Fm, VRR, contraction, HRR)
+   double *sgeo;              // [nshell][6] A - B and C - D, written by the primitive kernel (null: each reader derives them)
    double *gscratch;          // HRR workspace in global memory for the largest classes
    int cls;                   // la*64 + lb*16 + lc*4 + ld
    int prim_variant;          // 0: k_prim3 where the class has it (lane per image); 1: k_prim2 (team per image)
-   int group_variant;         // 0: k_group3 where the class has it (lane per row); 1: k_group (warp per row)
+   int group_variant;         // 0: k_group3 where the class has it (lane per row), else k_group_mm (block per group); 1: k_group (warp per row)
 };
 
 bool build_class_plan(int la, int lb, int lc, int ld, ClassPlan &p);
@@ -78,12 +79,6 @@ size_t group_global_scratch(const ClassPlan &hp, int *grid, int *warps);
 constexpr int kGroupShellCacheDoubles = 16;
 constexpr int kGroupKpDoubles = 32 + kGroupShellCacheDoubles;
 constexpr int kGroupRowsPerWarp = 4;      // consecutive rows a warp of k_group takes at a time
-// k_group_block: 128 threads share one row's workspace, 256 from this workspace size on (on the
-// 64-molecule l <= 3 workload the wider block was faster from about here on)
-constexpr int kGroupBlockWideDoubles = 6000;
-// k_group_block (variant 0) for the classes whose workspace holds at least this many doubles: on
-// the 64-molecule l <= 3 workload it was faster than one warp per row from about here on
-constexpr int kGroupBlockMinDoubles = 1536;
 int prim_team_size(const ClassPlan &hp);
 // Incremental replay screening (k_group_screen): mode 0 writes each group's largest |P| over the P
 // blocks its rows read into pmax (the recording's P); mode 1 sets flags[g] = 0 for the groups whose
@@ -111,7 +106,7 @@ constexpr size_t kNoAllocScratchDoubles = (size_t)8 * 1024 * 1024;   // 64 MiB
 constexpr int kMaxDevices = 64;
 cudaError_t noalloc_scratch(double **ptr);
 // loads every kernel on the current device (once per device, from libgint_init)
-cudaError_t preload_kernels();
+cudaError_t preload_kernels(const double *c2s_l0to3);
 // sustained FP64 FMA rate of this GPU (TFLOP/s), from a dependent-FMA kernel
 double measure_fp64_peak_tflops();
 

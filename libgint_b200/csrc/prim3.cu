@@ -64,6 +64,7 @@ k_prim3(DevCtx ctx, BatchArgs bt, int cp) {
    extern __shared__ __align__(16) double smem[];
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
    const int Ng = ctx.Ng;
+   write_shell_vectors(ctx, bt);
    // the image vectors in order of length, shared by the block
    double4 *simg = reinterpret_cast<double4 *>(smem);
    for (int i = threadIdx.x; i < 4 * Ng; i += blockDim.x) smem[i] = __ldg(reinterpret_cast<const double *>(ctx.img) + i);

@@ -97,6 +97,38 @@ static __device__ __forceinline__ void shell_geom(const DevCtx &ctx, const Basis
    }
 }
 
+// The HRR displacements A - B and C - D of one shell quartet.
+static __device__ __forceinline__ void shell_vectors(const DevCtx &ctx, const ShellRec &sh, double *v) {
+   const BasisEnt ea = ctx.ents[sh.ent[0]], eb = ctx.ents[sh.ent[1]], ec = ctx.ents[sh.ent[2]], ed = ctx.ents[sh.ent[3]];
+   double A[3], B[3], C[3], D[3], CDs[3];
+   shell_geom(ctx, ea, eb, ec, ed, sh.n1, sh.n2, A, B, C, D, CDs);
+   for (int q = 0; q < 3; q++) { v[q] = A[q] - B[q]; v[3 + q] = C[q] - D[q]; }
+}
+
+// The primitive kernels write them for every shell quartet of the segment, each once: a group kernel
+// needs them once per contraction row and tile, at the end of a chain of dependent loads.
+static __device__ __forceinline__ void write_shell_vectors(const DevCtx &ctx, const BatchArgs &bt) {
+   if (!bt.sgeo) return;
+   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < bt.nshell; i += gridDim.x * blockDim.x) {
+      double v[6];
+      shell_vectors(ctx, bt.shells[i], v);
+      double2 *o = reinterpret_cast<double2 *>(bt.sgeo + (size_t)6 * i);
+      o[0] = make_double2(v[0], v[1]); o[1] = make_double2(v[2], v[3]); o[2] = make_double2(v[4], v[5]);
+   }
+}
+
+// Shell quartet i's displacements for a group kernel.
+static __device__ __forceinline__ void read_shell_vectors(const DevCtx &ctx, const BatchArgs &bt, uint32_t i,
+                                                          const ShellRec &sh, double *v) {
+   if (bt.sgeo) {
+      const double2 *o = reinterpret_cast<const double2 *>(bt.sgeo + (size_t)6 * i);
+      const double2 x = __ldg(o), y = __ldg(o + 1), z = __ldg(o + 2);
+      v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y; v[4] = z.x; v[5] = z.y;
+   } else {
+      shell_vectors(ctx, sh, v);
+   }
+}
+
 // Per-primitive-quartet quantities shared by every image n3. D = P - Q is rounded as the
 // reference's T formula rounds it; upper, lower, X2 and i2 (the truncation bounds and the
 // second patch coordinate, which depend on R only) are evaluated exactly as t_c_g0_n does.
@@ -392,6 +424,18 @@ static __device__ __forceinline__ SegSum<R> make_segsum(int key, int lane, R *ds
    sg.head = key >= 0 && (lane == 0 || kp != key);
    sg.dst = dst;
    return sg;
+}
+
+// whether the four P/K blocks that a row reads and updates lie inside the arrays
+static __device__ __forceinline__ bool row_in_range(const QrttRec &k, int na, int nb, int nc, int nd, size_t n) {
+   const int nx[4] = {na, na, nb, nb}, ny[4] = {nc, nd, nc, nd};
+   bool ok = true;
+#pragma unroll
+   for (int u = 0; u < 4; u++) {
+      const bool T = (k.T >> u) & 1;
+      ok = ok && (size_t)k.off[u] + (T ? (nx[u] - 1) * (int)k.ld[u] + ny[u] - 1 : (ny[u] - 1) * (int)k.ld[u] + nx[u] - 1) < n;
+   }
+   return ok;
 }
 
 // fm_eval_geo for the FP32 path: the same decisions (truncation, branch, patch) in FP64, the
