@@ -1,5 +1,5 @@
 // group3.cu -- k_group3<la,lb,lc,ld>: contraction + HRR + image-pair sum + spherical transform +
-// K update, one lane per contraction row, for the classes with generated HRR code (grp_gen.cuh).
+// K update, one lane (or four) per contraction row, for the classes with generated HRR code (grp_gen.cuh).
 //
 // A group is one set quartet of one class: all its image pairs (shell quartets) and its
 // nla*nlb*nlc*nld contraction rows. One lane takes one row: it contracts the image-summed targets
@@ -120,17 +120,23 @@ struct Group3Shape {
 
 // R = double: the FP64 path; R = float: the FP32 path (contraction, HRR and spherical transform in
 // FP32 from the FP32 targets of k_prim3; the K update in FP64).
-template <int LA, int LB, int LC, int LD, class R>
+// TPR lanes share one contraction row: they divide its primitives, add their targets up, and all go on
+// with the sums.
+template <int LA, int LB, int LC, int LD, class R, int TPR>
 __global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB) k_group3(DevCtx ctx, BatchArgs bt) {
    using G = GrpGen<LA, LB, LC, LD>;
    constexpr int S = G::S, Nc = G::Nc, Ns = G::Ns;
    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-   const uint32_t nblk = (bt.nqrtt + 31) >> 5;
-   // one lane per contraction row: a warp takes 32 consecutive rows, so the lanes of one set
-   // quartet's rows read the same primitive codes and image-summed targets (broadcast loads)
+   constexpr int RPW = 32 / TPR;   // rows a warp
+   const uint32_t nblk = (bt.nqrtt + RPW - 1) / RPW;
+   const int sub = lane % TPR;
+   const unsigned team = TPR == 1 ? 1u << lane : ((1u << TPR) - 1u) << (lane - sub);
+   // a warp takes RPW consecutive rows, so the lanes of one set quartet's rows read the same
+   // primitive codes and image-summed targets (broadcast loads)
    for (uint32_t blk = blockIdx.x * wpb + (threadIdx.x >> 5); blk < nblk; blk += gridDim.x * wpb) {
-      const uint32_t q0 = blk << 5, q = q0 + lane;
-      const uint32_t gi = row_group_warp(bt, q0, lane);
+      const uint32_t q0 = blk * RPW, q = q0 + lane / TPR;
+      uint32_t gi = row_group_warp(bt, q0 & ~31u, lane);
+      if (TPR > 1) gi = __shfl_sync(0xffffffffu, gi, (int)(q0 & 31u) + lane / TPR);
       if (q >= bt.nqrtt || (bt.gflags && !__ldg(bt.gflags + gi))) continue;   // screened (incremental)
       const GroupRec Gr = bt.groups[gi];
       const int nl1 = Gr.nl[1], nl2 = Gr.nl[2], nl3 = Gr.nl[3];
@@ -154,7 +160,7 @@ __global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB) k_grou
          // contraction over the primitives (reference src/compute_ECO.cpp:131-212); four per
          // iteration so that the next ones' loads overlap this one's FMAs
 #pragma unroll 4
-         for (uint32_t ip = 0; ip < sh.nprm; ip++) {
+         for (uint32_t ip = sub; ip < sh.nprm; ip += TPR) {
             const uint32_t code = __ldg(bt.prm + sh.prm_off + ip);
             const R kp = (R)__ldg(Ka + (code >> 24)) * (R)__ldg(Kb + ((code >> 16) & 255)) *
                          (R)__ldg(Kc + ((code >> 8) & 255)) * (R)__ldg(Kd + (code & 255));
@@ -162,11 +168,16 @@ __global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB) k_grou
 #pragma unroll
             for (int j = 0; j < S; j++) T[j] += kp * __ldg(row + j);
          }
+#pragma unroll
+         for (int o = 1; o < TPR; o <<= 1)
+#pragma unroll
+            for (int j = 0; j < S; j++) T[j] += __shfl_xor_sync(team, T[j], o);
          double v[6];
          read_shell_vectors(ctx, bt, Gr.shell_off + s, sh, v);
          const R AB[3] = {(R)v[0], (R)v[1], (R)v[2]}, CD[3] = {(R)v[3], (R)v[4], (R)v[5]};
          G::hrr(T, AB, CD, cart);
       }
+      if (TPR > 1 && sub) continue;
       R sph[Ns];
       G::sph(cart, sph);
       const QrttRec k = bt.qrtts[q];
@@ -180,22 +191,33 @@ __global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB) k_grou
    }
 }
 
-template <int LA, int LB, int LC, int LD>
-cudaError_t launch_one(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st) {
+template <int LA, int LB, int LC, int LD, int TPR>
+cudaError_t launch_lanes(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st) {
    const int threads = 128;
-   // one 32-row block per warp: rows cost from one primitive to thousands, so the block scheduler,
-   // which starts a new block wherever one finishes, balances them better than a grid-stride loop
-   const long blocks = std::max(1L, std::min(((long)bt.nqrtt + threads - 1) / threads, 1L << 30));
+   // 32 / TPR rows per warp: rows cost from one primitive to thousands, so the block scheduler, which
+   // starts a new block wherever one finishes, balances them better than a grid-stride loop
+   const long blocks = std::max(1L, std::min(((long)bt.nqrtt * TPR + threads - 1) / threads, 1L << 30));
    if constexpr (class_has_fp32(LA, LB, LC, LD)) {
       if (bt.fp32) {
-         k_group3<LA, LB, LC, LD, float><<<(unsigned)blocks, threads, 0, st>>>(ctx, bt);
+         k_group3<LA, LB, LC, LD, float, TPR><<<(unsigned)blocks, threads, 0, st>>>(ctx, bt);
          return cudaGetLastError();
       }
    } else {
       if (bt.fp32) return cudaErrorInvalidValue;   // no FP32 segments for these classes
    }
-   k_group3<LA, LB, LC, LD, double><<<(unsigned)blocks, threads, 0, st>>>(ctx, bt);
+   k_group3<LA, LB, LC, LD, double, TPR><<<(unsigned)blocks, threads, 0, st>>>(ctx, bt);
    return cudaGetLastError();
+}
+
+template <int LA, int LB, int LC, int LD>
+cudaError_t launch_one(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st) {
+   // Too few rows to fill half of the warps that the registers leave room for: four lanes a row. (The
+   // rows of one set quartet read the same targets, so more lanes a row cost reads where there are
+   // rows enough: the line lies where the GPU has nothing else to run.) The classes of L <= 3, kernels one
+   // after another: 4 molecules l <= 2 2.70 -> 0.97 ms, 24 clusters 6.85 -> 2.93 ms, 32 molecules
+   // l <= 2 2.83 -> 1.38 ms; the 1/4096 sample of 64 molecules, with 150k rows and more a class, unchanged.
+   if (bt.nqrtt < 148u * 64 * Group3Shape<LA, LB, LC, LD>::MINB) return launch_lanes<LA, LB, LC, LD, 4>(ctx, bt, st);
+   return launch_lanes<LA, LB, LC, LD, 1>(ctx, bt, st);
 }
 
 template <int I>
@@ -222,12 +244,14 @@ struct PartPreload {
          return cudaSuccess;
       } else {
          constexpr int c = kGrpGenClasses[I];
+         constexpr int la = (c >> 6) & 3, lb = (c >> 4) & 3, lc = (c >> 2) & 3, ld = c & 3;
          cudaFuncAttributes a;
-         cudaError_t e = cudaFuncGetAttributes(&a, k_group3<(c >> 6) & 3, (c >> 4) & 3, (c >> 2) & 3, c & 3, double>);
-         if (e != cudaSuccess) return e;
-         if constexpr (class_has_fp32((c >> 6) & 3, (c >> 4) & 3, (c >> 2) & 3, c & 3)) {
-            e = cudaFuncGetAttributes(&a, k_group3<(c >> 6) & 3, (c >> 4) & 3, (c >> 2) & 3, c & 3, float>);
-            if (e != cudaSuccess) return e;
+         cudaError_t e;
+         if ((e = cudaFuncGetAttributes(&a, k_group3<la, lb, lc, ld, double, 1>)) != cudaSuccess) return e;
+         if ((e = cudaFuncGetAttributes(&a, k_group3<la, lb, lc, ld, double, 4>)) != cudaSuccess) return e;
+         if constexpr (class_has_fp32(la, lb, lc, ld)) {
+            if ((e = cudaFuncGetAttributes(&a, k_group3<la, lb, lc, ld, float, 1>)) != cudaSuccess) return e;
+            if ((e = cudaFuncGetAttributes(&a, k_group3<la, lb, lc, ld, float, 4>)) != cudaSuccess) return e;
          }
          return PartPreload<I + kGroup3Parts>::run();
       }
