@@ -650,8 +650,9 @@ cudaError_t launch_prim(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan 
    if (bt.fp32) return cudaErrorInvalidValue;   // FP32 segments exist only for classes with k_prim3
    // a chunk is as large as gives every resident team one, within what fills a G_m batch (about four
    // pairs a primitive with images, one without) and kPrim2Chunk; where the VRR is the larger part
-   // of a primitive's time the lanes of G_m matter less than a finer split
-   const int fill = (hp.V >= 1000 ? 2 : 4) * (ctx.Ng == 1 ? 2 : 1);
+   // of a primitive's time the lanes of G_m matter less than a finer split, and with fewer
+   // primitives than four an SM nothing but the longest team counts
+   const int fill = bt.nprm < 148u * 4 ? 1 : (hp.V >= 1000 ? 2 : 4) * (ctx.Ng == 1 ? 2 : 1);
    auto chunk = [&](long teams) { return (int)std::max((long)fill, std::min((long)kPrim2Chunk, ((long)bt.nprm + teams - 1) / teams)); };
    const size_t plan_bytes = (size_t)plan_smem_doubles() * 8;
    int cp = chunk(148 * 14);
@@ -661,7 +662,7 @@ cudaError_t launch_prim(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan 
       nchunk = ((long)bt.nprm + cp - 1) / cp;
       const size_t wd = prim2_team_doubles(hp, cp), smem = plan_bytes + wd * 8;
       const unsigned blocks = (unsigned)std::min(nchunk, 148L * 64);
-      if (hp.V >= kPrim2WideDoubles) k_prim2<256><<<blocks, 256, smem, st>>>(ctx, bt, cp, (int)wd);
+      if (hp.V >= kPrim2WideDoubles || (hp.V >= 1000 && nchunk < 148)) k_prim2<256><<<blocks, 256, smem, st>>>(ctx, bt, cp, (int)wd);
       else k_prim2<128><<<blocks, 128, smem, st>>>(ctx, bt, cp, (int)wd);
       return cudaGetLastError();
    }

@@ -244,10 +244,10 @@ cudaError_t launch_one(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st) 
    const int maxw = Sh::THREADS / 32;
    const int nwmax = (int)std::max<size_t>(1, std::min<size_t>(maxw, (budget - std::min(budget, neigh_bytes)) / warp_bytes));
    // A segment too small to give every resident warp CP primitives is cut finer, but not below what
-   // fills a G_m batch (one pair each without images, about four each with them), and it is spread
-   // over the SMs before a block takes more warps.
+   // fills a G_m batch (one pair each without images, about four each with them) unless it is too
+   // small for one such chunk an SM; and it is spread over the SMs before a block takes more warps.
    const long slots = 148L * Sh::MINB * nwmax;
-   const int cpmin = ctx.Ng == 1 ? Sh::CP : std::min(8, Sh::CP);
+   const int cpmin = ctx.Ng == 1 ? Sh::CP : std::min(bt.nprm < 148u * 8 ? 2 : 8, Sh::CP);
    const int cp = (int)std::max((long)cpmin, std::min((long)Sh::CP, ((long)bt.nprm + slots - 1) / slots));
    const long nchunk = ((long)bt.nprm + cp - 1) / cp;
    const int nw = (int)std::max(1L, std::min((long)nwmax, (nchunk + 147) / 148));
