@@ -554,6 +554,9 @@ static cudaStream_t worker_for(Handle *h, int i, bool uses_scratch) {
 // Doubles from a segment's image-summed targets to its shell quartets' displacements (BatchArgs::sgeo).
 static size_t sgeo_offset(Handle *h, int c, size_t nprm) { return (nprm * h->plans[c & 255].S + 3) & ~(size_t)3; }
 
+// Doubles of global HRR scratch that a class's group kernel may use.
+static size_t scratch_of(const ClassPlan &hp) { int a = 0, b = 0; return group_global_scratch(hp, &a, &b); }
+
 // The worker stream (index) that a replay gives its i-th recorded segment (of class c), as
 // worker_for does, and the image-summed targets and displacements that segment needs (doubles,
 // 32-byte multiple).
@@ -1850,35 +1853,64 @@ int libgint_replay_noalloc(void *hh, const double *P_dev, double *K_dev, size_t 
    ctx.FP_size = K_size;
    ctx.cnt = nullptr;
    if (!ck(h, cudaMemsetAsync(K_dev, 0, K_size * 8, st), "libgint_replay_noalloc: K zero")) return h->err;
-   for (auto &rb : h->recs) {
+   // One segment's two kernels on stream s, with its intermediates in scr[0, room).
+   auto run = [&](const Handle::RecBatch &rb, const Handle::RecSeg &g, double *at, size_t room, cudaStream_t s) {
       char *base = (char *)rb.rec.p;
+      const ClassPlan &hp = h->plans[g.c & 255];
+      BatchArgs bt;
+      std::memset(&bt, 0, sizeof(bt));
+      bt.cls = g.c & 255;
+      bt.fp32 = g.c >= kFp32;
+      bt.prim_variant = h->tune_prim[g.c & 255];
+      bt.group_variant = h->tune_group[g.c & 255];
+      bt.plan = (const ClassPlan *)h->d_plans.p + (g.c & 255);
+      bt.prm = (const uint32_t *)(base + g.o_prm);
+      bt.prm_shell = (const uint32_t *)(base + g.o_ps);
+      bt.shells = (const ShellRec *)(base + g.o_sh);
+      bt.groups = (const GroupRec *)(base + g.o_g);
+      bt.qrtts = (const QrttRec *)(base + g.o_q);
+      bt.rowgrp = (const uint32_t *)(base + g.o_rg);
+      bt.nprm = g.nprm; bt.nshell = g.nshell; bt.ngroup = g.ngroup; bt.nqrtt = g.nqrtt;
+      bt.AC = at;
+      const size_t gs0 = ((size_t)g.nprm * hp.S + 31) & ~(size_t)31;
+      bt.gscratch = at + gs0;
+      const size_t sg0 = gs0 + ((scratch_of(hp) + 3) & ~(size_t)3);
+      if (sg0 + (size_t)6 * g.nshell <= room) bt.sgeo = at + sg0;   // else derived by their readers
+      return ck(h, launch_prim(ctx, bt, hp, s), "libgint_replay_noalloc: k_prim launch") &&
+             ck(h, launch_group(ctx, bt, hp, s), "libgint_replay_noalloc: k_group launch");
+   };
+   // The segments that fit a share of the scratch run on the worker streams, each stream in its
+   // own share, as the ordinary replay does: a small system's segments are far too small to fill the
+   // GPU one after another (4 molecules, 81 classes: 3.5 ms in a row, 0.68 ms so). The others follow on the
+   // caller's stream, one after another in the whole scratch. A stream being captured keeps to itself.
+   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+   if (!ck(h, cudaStreamIsCapturing(st, &cap), "libgint_replay_noalloc: capture status")) return h->err;
+   const size_t share = (kNoAllocScratchDoubles / kWorkStreams) & ~(size_t)31;
+   auto small = [&](const Handle::RecSeg &g) {
+      const ClassPlan &hp = h->plans[g.c & 255];
+      return cap == cudaStreamCaptureStatusNone && (((size_t)g.nprm * hp.S + 31) & ~(size_t)31) + scratch_of(hp) <= share;
+   };
+   bool ok = true;
+   int n = 0;
+   for (auto &rb : h->recs)
       for (auto &g : rb.segs) {
-         const ClassPlan &hp = h->plans[g.c & 255];
-         BatchArgs bt;
-         std::memset(&bt, 0, sizeof(bt));
-         bt.cls = g.c & 255;
-         bt.fp32 = g.c >= kFp32;
-         bt.prim_variant = h->tune_prim[g.c & 255];
-         bt.group_variant = h->tune_group[g.c & 255];
-         bt.plan = (const ClassPlan *)h->d_plans.p + (g.c & 255);
-         bt.prm = (const uint32_t *)(base + g.o_prm);
-         bt.prm_shell = (const uint32_t *)(base + g.o_ps);
-         bt.shells = (const ShellRec *)(base + g.o_sh);
-         bt.groups = (const GroupRec *)(base + g.o_g);
-         bt.qrtts = (const QrttRec *)(base + g.o_q);
-         bt.rowgrp = (const uint32_t *)(base + g.o_rg);
-         bt.nprm = g.nprm; bt.nshell = g.nshell; bt.ngroup = g.ngroup; bt.nqrtt = g.nqrtt;
-         bt.AC = scr;                                                   // segments run in stream order
-         const size_t gs0 = ((size_t)g.nprm * hp.S + 31) & ~(size_t)31;
-         bt.gscratch = scr + gs0;
-         int ga = 0, gb = 0;
-         const size_t sg0 = gs0 + ((group_global_scratch(hp, &ga, &gb) + 3) & ~(size_t)3);
-         if (sg0 + (size_t)6 * g.nshell <= kNoAllocScratchDoubles) bt.sgeo = scr + sg0;   // else derived by their readers
-         if (!ck(h, launch_prim(ctx, bt, hp, st), "libgint_replay_noalloc: k_prim launch")) return h->err;
-         if (!ck(h, launch_group(ctx, bt, hp, st), "libgint_replay_noalloc: k_group launch")) return h->err;
+         if (!ok || !small(g)) continue;
+         if (n == 0) {
+            ok = ck(h, cudaEventRecord(h->fork_ev, st), "libgint_replay_noalloc: event record");
+            for (int w = 0; ok && w < kWorkStreams; w++)
+               ok = ck(h, cudaStreamWaitEvent(h->work[w], h->fork_ev, 0), "libgint_replay_noalloc: stream wait");
+            if (!ok) break;
+         }
+         const int w = n++ % kWorkStreams;
+         ok = run(rb, g, scr + (size_t)w * share, share, h->work[w]);
       }
-   }
-   return 0;
+   for (int w = 0; n && w < kWorkStreams; w++)
+      ok = ck(h, cudaEventRecord(h->work_ev[w], h->work[w]), "libgint_replay_noalloc: event record") &&
+           ck(h, cudaStreamWaitEvent(st, h->work_ev[w], 0), "libgint_replay_noalloc: stream wait") && ok;
+   for (auto &rb : h->recs)
+      for (auto &g : rb.segs)
+         if (ok && !small(g)) ok = run(rb, g, scr, kNoAllocScratchDoubles, st);
+   return h->err;
 }
 
 // the same with the summed device time of each kernel kind: kt[0] = k_prim, kt[1] = k_group
