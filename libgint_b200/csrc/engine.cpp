@@ -15,6 +15,8 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -277,6 +279,8 @@ struct Handle {
    bool basis_dirty = true, ent_dirty = true;
    // device-resident data
    DBuf d_pool, d_ents, d_neighs, d_img, d_C0, d_C0f, d_lut, d_bw, d_ft, d_plans, d_err, d_vops, d_tmap;
+   char *stage = nullptr;           // pinned chunks of staged_copy
+   cudaEvent_t stage_ev[8] = {};
    DBuf d_tmax;                     // incremental replays: tile maxima of |dP|
    std::vector<VOp> vops;           // precompiled VRR instructions of all classes
    std::vector<uint16_t> tmap;      // and the workspace elements of their targets
@@ -425,6 +429,72 @@ static std::vector<double4> images_by_length(const std::vector<double> &neighs) 
    }
    std::stable_sort(v.begin(), v.end(), [](const double4 &a, const double4 &b) { return a.w < b.w; });
    return v;
+}
+
+// Copies a large P or K between the caller's pageable array and the device through pinned memory,
+// kStageThreads threads at it, each with kStageSlots chunks of its own in turn: one thread's memcpy
+// moves about 13 GB/s, a third of what the link takes, and so did cudaMemcpy on the array itself
+// (51 MB: 4.0 ms each way). Like it, the call returns when the caller's array may be used again
+// (up: after its chunks were read; the device copies are on the handle's stream).
+constexpr int kStageThreads = 4, kStageSlots = 2;
+constexpr size_t kStageChunk = (size_t)1 << 20, kStageMin = (size_t)8 << 20;
+
+static bool staged_copy(Handle *h, void *dev, void *host, size_t bytes, bool up, const char *what) {
+   const cudaMemcpyKind kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+   constexpr int nslot = kStageThreads * kStageSlots;
+   // only pageable memory gains: pinned memory is copied at the link's rate as it is
+   cudaPointerAttributes at;
+   bool stage = bytes >= kStageMin;
+   if (stage && cudaPointerGetAttributes(&at, host) != cudaSuccess) { cudaGetLastError(); stage = false; }
+   stage = stage && at.type == cudaMemoryTypeUnregistered;
+   if (stage && !h->stage) {
+      if (cudaHostAlloc((void **)&h->stage, nslot * kStageChunk, cudaHostAllocPortable) != cudaSuccess) {
+         cudaGetLastError();   // no pinned memory to be had: the plain copy below
+         h->stage = nullptr;
+      }
+      for (auto &e : h->stage_ev)
+         if (h->stage && !e && !ck(h, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), what)) return false;
+   }
+   if (!stage || !h->stage)
+      return ck(h, cudaMemcpyAsync(up ? dev : host, up ? host : dev, bytes, kind, h->stream), what) &&
+             (up || ck(h, cudaStreamSynchronize(h->stream), what));
+   const size_t nchunk = (bytes + kStageChunk - 1) / kStageChunk;
+   cudaError_t err[kStageThreads];
+   auto work = [&](int t) {
+      cudaError_t e = cudaSetDevice(h->device);
+      auto slot = [&](size_t i) { return t * kStageSlots + (int)((i / kStageThreads) % kStageSlots); };
+      auto len = [&](size_t i) { return std::min(kStageChunk, bytes - i * kStageChunk); };
+      auto start = [&](size_t i) {   // chunk i's device copy
+         char *p = h->stage + slot(i) * kStageChunk, *d = (char *)dev + i * kStageChunk;
+         if (e == cudaSuccess) e = cudaMemcpyAsync(up ? d : p, up ? p : d, len(i), kind, h->stream);
+         if (e == cudaSuccess) e = cudaEventRecord(h->stage_ev[slot(i)], h->stream);
+      };
+      if (!up)
+         for (int k = 0; k < kStageSlots; k++)
+            if (t + (size_t)k * kStageThreads < nchunk) start(t + (size_t)k * kStageThreads);
+      for (size_t i = t; i < nchunk && e == cudaSuccess; i += kStageThreads) {
+         // up: the slot's previous copy has left it; down: this chunk's has arrived
+         if (e == cudaSuccess) e = cudaEventSynchronize(h->stage_ev[slot(i)]);
+         if (e != cudaSuccess) break;
+         char *p = h->stage + slot(i) * kStageChunk, *u = (char *)host + i * kStageChunk;
+         std::memcpy(up ? p : u, up ? u : p, len(i));
+         if (up) start(i);
+         else if (i + (size_t)kStageSlots * kStageThreads < nchunk) start(i + (size_t)kStageSlots * kStageThreads);
+      }
+      err[t] = e;
+   };
+   std::thread th[kStageThreads];
+   for (int t = 1; t < kStageThreads; t++) {
+      try { th[t] = std::thread(work, t); } catch (const std::system_error &) {}   // no thread: its share below
+   }
+   work(0);
+   for (int t = 1; t < kStageThreads; t++) {
+      if (th[t].joinable()) th[t].join();
+      else work(t);
+   }
+   for (cudaError_t e : err)
+      if (!ck(h, e, what)) { cudaStreamSynchronize(h->stream); return false; }
+   return true;
 }
 
 static bool upload_tables(Handle *h) {
@@ -786,7 +856,7 @@ static void set_P_impl(Handle *h, int nspin, const double *Pa, const double *Pb,
       bool good = ok && !h->err;
       for (int sp = 0; good && sp < nspin; sp++) {
          good = ensure(h, t->P[sp], (size_t)n * 8, "P") && ensure(h, t->K[sp], (size_t)n * 8, "K") &&
-                h2d(h, t->P[sp].p, src[sp], (size_t)n * 8, "P upload") &&
+                staged_copy(h, t->P[sp].p, const_cast<double *>(src[sp]), (size_t)n * 8, true, "P upload") &&
                 ck(h, cudaMemsetAsync(t->K[sp].p, 0, (size_t)n * 8, h->stream), "K zero");
          if (good) h->h2d_bytes += (long long)n * 8;
       }
@@ -821,7 +891,7 @@ static void get_K_impl(Handle *h, double *Ka, double *Kb) {
       if (have) {
          double *dst[2] = {Ka, Kb};
          for (int sp = 0; sp < h->nspin; sp++)
-            if (dst[sp]) ck(h, cudaMemcpy(dst[sp], h->team->K[sp].p, h->FP_size * 8, cudaMemcpyDeviceToHost), "K download");
+            if (dst[sp]) staged_copy(h, h->team->K[sp].p, dst[sp], h->FP_size * 8, false, "K download");
       }
    }
 }
@@ -838,7 +908,7 @@ static void set_K_impl(Handle *h, int nspin, const double *Ka, const double *Kb,
    {
       if (ok) {
          const double *src[2] = {Ka, Kb};
-         for (int sp = 0; sp < nspin; sp++) h2d(h, h->team->K[sp].p, src[sp], (size_t)K_size * 8, "K upload");
+         for (int sp = 0; sp < nspin; sp++) staged_copy(h, h->team->K[sp].p, const_cast<double *>(src[sp]), (size_t)K_size * 8, true, "K upload");
          ck(h, cudaStreamSynchronize(h->stream), "K upload");
       }
    }
@@ -2062,6 +2132,8 @@ void libgint_destroy_handle(void *hh) {
                    &h->d_plans, &h->d_err};
    for (DBuf *b : bufs) release(*b);
    h->team.reset();
+   if (h->stage) cudaFreeHost(h->stage);
+   for (auto &e : h->stage_ev) if (e) cudaEventDestroy(e);
    for (int w = 0; w < kWorkStreams; w++) {
       if (h->work[w]) cudaStreamDestroy(h->work[w]);
       if (h->work_ev[w]) cudaEventDestroy(h->work_ev[w]);
