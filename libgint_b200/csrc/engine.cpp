@@ -243,12 +243,18 @@ struct Slot {
    bool busy = false, copy_busy = false;
 };
 
-// Class segments of one batch are independent (K is updated with atomics), so they run on
-// kWorkStreams worker streams that fork from and join back to the handle's stream; the tails of
-// one class's kernels then overlap the next class's. Six workers (seven streams with the handle's,
-// within the runtime's default eight device connections) replay the 32-water K build 2% faster
-// than four; eight or twelve gain nothing more.
-constexpr int kWorkStreams = 6;
+// Class segments of one batch are independent (K is updated with atomics), so they run on worker
+// streams that fork from and join back to the handle's stream; the tails of one class's kernels then
+// overlap the next class's, and the classes of a small system run beside each other. Replays of small
+// systems gain up to here (4 molecules l <= 2: 0.68 ms with 6 streams, 0.35 with 16; 2 molecules
+// l <= 3: 5.3 and 2.4 ms); 32 molecules l <= 2 and more fill the GPU with 6.
+constexpr int kWorkStreams = 16;
+constexpr int kFewWorkStreams = 6;
+// All of them for segments of fewer primitives than this on average: 24 clusters, 8.6k a segment, gain
+// 7 % from 16 streams, 32 molecules l <= 2, 34k, lose 3 % (and each stream of a replay has its own
+// buffer of image-summed targets).
+constexpr size_t kManyStreamsPrims = 16384;
+static bool many_streams(size_t prims, size_t segments) { return prims < segments * kManyStreamsPrims; }
 
 struct Handle {
    int device = 0;
@@ -320,11 +326,12 @@ struct Handle {
    std::vector<RecBatch> recs;
    long long rec_gen = 0;           // bumped whenever the recording changes
    // the replay captured as a CUDA graph, and what it was captured with
-   struct GraphKey { DevCtx ctx; long long rec_gen; void *ac, *gscr; size_t half; double eps; };
+   struct GraphKey { DevCtx ctx; long long rec_gen; void *ac, *gscr; size_t half; double eps; int streams; };
    cudaGraphExec_t graph_exec = nullptr;
    GraphKey graph_key;
    long long graph_launches = 0;
    DBuf rec_ac, rec_gscr;
+   int replay_streams = kFewWorkStreams;  // worker streams of the replay (prepare_replay)
    size_t arena_off[kWorkStreams] = {};   // replay: each worker stream's AC arena in rec_ac (doubles)
    // optional device event counters [256 classes][4]
    DBuf d_cnt;
@@ -601,39 +608,35 @@ static void ensure_ent_base(Handle *h) {
    h->ent_dirty = false;
 }
 
-// worker streams wait for everything queued so far on the handle's stream
-static void fork_workers(Handle *h) {
+// the first n worker streams wait for everything queued so far on the handle's stream
+static void fork_workers(Handle *h, int n) {
    ck(h, cudaEventRecord(h->fork_ev, h->stream), "event record");
-   for (int w = 0; w < kWorkStreams; w++) ck(h, cudaStreamWaitEvent(h->work[w], h->fork_ev, 0), "stream wait");
+   for (int w = 0; w < n; w++) ck(h, cudaStreamWaitEvent(h->work[w], h->fork_ev, 0), "stream wait");
 }
 
-// the handle's stream waits for everything queued on the worker streams
-static void join_workers(Handle *h) {
-   for (int w = 0; w < kWorkStreams; w++) {
+// the handle's stream waits for everything queued on them
+static void join_workers(Handle *h, int n) {
+   for (int w = 0; w < n; w++) {
       ck(h, cudaEventRecord(h->work_ev[w], h->work[w]), "event record");
       ck(h, cudaStreamWaitEvent(h->stream, h->work_ev[w], 0), "stream wait");
    }
 }
 
-// The worker stream of the i-th segment of a batch. Segments whose group kernel uses the shared
-// global HRR scratch all go to worker 0, so they never run concurrently.
-static cudaStream_t worker_for(Handle *h, int i, bool uses_scratch) {
-   return uses_scratch ? h->work[0] : h->work[1 + i % (kWorkStreams - 1)];
-}
-
 // Doubles from a segment's image-summed targets to its shell quartets' displacements (BatchArgs::sgeo).
 static size_t sgeo_offset(Handle *h, int c, size_t nprm) { return (nprm * h->plans[c & 255].S + 3) & ~(size_t)3; }
 
-// Doubles of global HRR scratch that a class's group kernel may use.
-static size_t scratch_of(const ClassPlan &hp) { int a = 0, b = 0; return group_global_scratch(hp, &a, &b); }
-
-// The worker stream (index) that a replay gives its i-th recorded segment (of class c), as
-// worker_for does, and the image-summed targets and displacements that segment needs (doubles,
-// 32-byte multiple).
-static int replay_worker(Handle *h, int c, int i) {
-   int a, b;
-   return group_global_scratch(h->plans[c & 255], &a, &b) != 0 ? 0 : 1 + i % (kWorkStreams - 1);
+// Doubles of global HRR scratch that the group kernel of queue class c uses: one warp per row, on the
+// classes whose workspace does not fit shared memory.
+static size_t scratch_of(Handle *h, int c) {
+   int a = 0, b = 0;
+   return c < kFp32 && h->tune_group[c] ? group_global_scratch(h->plans[c], &a, &b) : 0;
 }
+
+// The worker stream (index) of the i-th segment of a batch or recording, of class c, among n. Segments
+// whose group kernel uses the global HRR scratch all go to worker 0, so they never run at once.
+static int worker_of(Handle *h, int c, int i, int n) { return scratch_of(h, c) != 0 ? 0 : 1 + i % (n - 1); }
+
+// The image-summed targets and displacements that a segment needs (doubles, 32-byte multiple).
 static size_t replay_seg_ac(Handle *h, int c, uint32_t nprm, uint32_t nshell) {
    return sgeo_offset(h, c, nprm) + (((size_t)6 * nshell + 3) & ~(size_t)3);
 }
@@ -760,7 +763,8 @@ static void flush(Handle *h) {
    ck(h, cudaEventRecord(s.ev_copy, h->stream), "event record");
    s.copy_busy = true;
    DevCtx ctx = make_ctx(h);
-   fork_workers(h);
+   const int nwork = std::min(many_streams(h->pend_prims, segs.size()) ? kWorkStreams : kFewWorkStreams, (int)segs.size() + 1);
+   fork_workers(h, nwork);
    int nseg = 0;
    for (const Seg &g : segs) {
       ClassQ &Q = h->q[g.c];
@@ -785,13 +789,12 @@ static void flush(Handle *h) {
       bt.nqrtt = (uint32_t)Q.qrtts.size();
       bt.AC = (double *)s.ac.p + g.ac_off;
       bt.sgeo = bt.AC + sgeo_offset(h, g.c, bt.nprm);
-      int gg = 0, gw = 0;
-      size_t gs = group_global_scratch(hp, &gg, &gw);
+      const size_t gs = scratch_of(h, g.c);
       if (gs) {
          if (!ensure(h, s.gscr, gs * 8, "HRR scratch")) return;
          bt.gscratch = (double *)s.gscr.p;
       }
-      cudaStream_t ws = worker_for(h, nseg++, gs != 0);
+      cudaStream_t ws = h->work[worker_of(h, g.c, nseg++, nwork)];
       if (!ck(h, launch_prim(ctx, bt, hp, ws), "k_prim launch")) return;
       if (!ck(h, launch_group(ctx, bt, hp, ws), "k_group launch")) return;
       h->n_launch += 2;
@@ -799,7 +802,7 @@ static void flush(Handle *h) {
       h->n_prims += bt.nprm; h->n_shells += bt.nshell; h->n_groups += bt.ngroup;
       if (bt.fp32) { h->n_prims_fp32 += bt.nprm; h->n_shells_fp32 += bt.nshell; }
    }
-   join_workers(h);
+   join_workers(h, nwork);
    ck(h, cudaEventRecord(s.ev, h->stream), "event record");
    s.busy = true;
    h->n_flush++;
@@ -935,7 +938,7 @@ static bool enqueue_replay(Handle *h, const DevCtx &ctx, std::vector<cudaEvent_t
       cudaEvent_t e; cudaEventCreate(&e); cudaEventRecord(e, h->stream); kev->push_back(e);
    };
    const bool spread = kev == nullptr;
-   if (spread) fork_workers(h);
+   if (spread) fork_workers(h, h->replay_streams);
    int nseg = 0;
    for (size_t bi = 0; bi < h->recs.size(); bi++) {
       auto &rb = h->recs[bi];
@@ -958,7 +961,7 @@ static bool enqueue_replay(Handle *h, const DevCtx &ctx, std::vector<cudaEvent_t
          bt.nprm = g.nprm; bt.nshell = g.nshell; bt.ngroup = g.ngroup; bt.nqrtt = g.nqrtt;
          // the segment's targets live in its worker stream's arena: the segments of one stream run
          // one after another, and no other stream touches that arena
-         const int w = replay_worker(h, g.c, nseg++);
+         const int w = worker_of(h, g.c, nseg++, h->replay_streams);
          bt.AC = (double *)h->rec_ac.p + h->arena_off[w];
          bt.sgeo = bt.AC + sgeo_offset(h, g.c, g.nprm);
          bt.gscratch = (double *)h->rec_gscr.p;
@@ -982,7 +985,7 @@ static bool enqueue_replay(Handle *h, const DevCtx &ctx, std::vector<cudaEvent_t
          *nlaunch += 2;
       }
    }
-   if (spread) join_workers(h);
+   if (spread) join_workers(h, h->replay_streams);
    return !h->err;
 }
 
@@ -997,26 +1000,42 @@ static void drop_graph(Handle *h) {
 // streams, with their batch-to-batch dependencies) and relaunched as one graph while the recording
 // and the device pointers it was captured with stay the same.
 // Checks that a replay can run and sizes its buffers; *half = the replay AC buffer's size (doubles).
-static bool prepare_replay(Handle *h, size_t *half) {
+// all_scratch: for either group kernel of every class (the autotuner runs both).
+static bool prepare_replay(Handle *h, size_t *half, bool all_scratch = false) {
    if (h->err) return false;
    use_device(h);
    if (h->recs.empty()) { set_error(h, 4, "libgint_replay: nothing recorded"); return false; }
    if (!h->team || !h->team->ok) { set_error(h, 4, "libgint_replay: call libgint_set_P first"); return false; }
    if (!upload_tables(h)) return false;
-   // The replay runs the recorded segments in order on the worker streams (replay_worker); the
-   // segments of one stream run one after another, so each stream needs one AC arena as large as
-   // the largest segment it runs, and the streams' arenas are disjoint.
-   size_t arena[kWorkStreams] = {}, gs = 0;
-   int i = 0;
+   // The replay runs the recorded segments in order on the worker streams (worker_of); the segments of
+   // one stream run one after another, so each stream needs one AC arena as large as the largest
+   // segment it runs, and the streams' arenas are disjoint. All streams are used for small segments
+   // (many_streams) where their arenas take no more than the few streams' do, or than an eighth of the
+   // work budget.
+   size_t gs = 0, ac = 0;
+   auto arenas = [&](int n) {
+      size_t arena[kWorkStreams] = {}, sum = 0;
+      int i = 0;
+      for (auto &rb : h->recs)
+         for (auto &g : rb.segs) {
+            const int w = worker_of(h, g.c, i++, n);
+            arena[w] = std::max(arena[w], replay_seg_ac(h, g.c, g.nprm, g.nshell));
+         }
+      for (int w = 0; w < n; w++) { h->arena_off[w] = sum; sum += arena[w]; }
+      return sum;
+   };
+   size_t prims = 0, segs = 0;
    for (auto &rb : h->recs)
       for (auto &g : rb.segs) {
-         const int w = replay_worker(h, g.c, i++);
-         arena[w] = std::max(arena[w], replay_seg_ac(h, g.c, g.nprm, g.nshell));
-         int a, b;
-         gs = std::max(gs, group_global_scratch(h->plans[g.c & 255], &a, &b));
+         int a = 0, b = 0;
+         prims += g.nprm;
+         segs++;
+         gs = std::max(gs, all_scratch ? group_global_scratch(h->plans[g.c & 255], &a, &b) : scratch_of(h, g.c));
       }
-   size_t ac = 0;
-   for (int w = 0; w < kWorkStreams; w++) { h->arena_off[w] = ac; ac += arena[w]; }
+   const size_t few = arenas(kFewWorkStreams), all = arenas(kWorkStreams);
+   h->replay_streams = many_streams(prims, segs) && all <= std::max(few, h->max_mem_mb * (size_t)(1 << 20) / 64)
+                           ? kWorkStreams : kFewWorkStreams;
+   ac = h->replay_streams == kWorkStreams ? all : arenas(kFewWorkStreams);
    if (!ensure(h, h->rec_ac, std::max<size_t>(ac * 8, 256), "replay AC")) return false;
    if (gs && !ensure(h, h->rec_gscr, gs * 8, "replay HRR scratch")) return false;
    *half = ac;
@@ -1057,7 +1076,7 @@ static double replay_impl(Handle *h, double *kt, double *kcls = nullptr, double 
       std::memset(&key, 0, sizeof(key));
       std::memcpy(&key.ctx, &ctx, sizeof(ctx));
       key.rec_gen = h->rec_gen;
-      key.ac = h->rec_ac.p; key.gscr = h->rec_gscr.p; key.half = ac; key.eps = eps;
+      key.ac = h->rec_ac.p; key.gscr = h->rec_gscr.p; key.half = ac; key.eps = eps; key.streams = h->replay_streams;
       if (!h->graph_exec || std::memcmp(&key, &h->graph_key, sizeof(key)) != 0) {
          drop_graph(h);
          cudaGraph_t graph = nullptr;
@@ -1206,7 +1225,7 @@ static void record_group_pmax(Handle *h) {
 // afterwards (the timing runs add into it).
 static int autotune_impl(Handle *h, int *out) {
    size_t ac = 0;
-   if (!prepare_replay(h, &ac)) return h->err ? h->err : 4;
+   if (!prepare_replay(h, &ac, true)) return h->err ? h->err : 4;
    drop_graph(h);
    DevCtx ctx = make_ctx(h);
    double t[256][2][2] = {};
@@ -1218,7 +1237,7 @@ static int autotune_impl(Handle *h, int *out) {
       auto &rb = h->recs[bi];
       char *base = (char *)rb.rec.p;
       for (auto &g : rb.segs) {
-         const int wk = replay_worker(h, g.c, nseg++);   // the arena the replay gives this segment
+         const int wk = worker_of(h, g.c, nseg++, h->replay_streams);   // the arena the replay gives this segment
          if (g.c >= kFp32) continue;
          const int c = g.c;
          const ClassPlan &hp = h->plans[c];
@@ -1944,22 +1963,28 @@ int libgint_replay_noalloc(void *hh, const double *P_dev, double *K_dev, size_t 
       bt.AC = at;
       const size_t gs0 = ((size_t)g.nprm * hp.S + 31) & ~(size_t)31;
       bt.gscratch = at + gs0;
-      const size_t sg0 = gs0 + ((scratch_of(hp) + 3) & ~(size_t)3);
+      const size_t sg0 = gs0 + ((scratch_of(h, g.c) + 3) & ~(size_t)3);
       if (sg0 + (size_t)6 * g.nshell <= room) bt.sgeo = at + sg0;   // else derived by their readers
       return ck(h, launch_prim(ctx, bt, hp, s), "libgint_replay_noalloc: k_prim launch") &&
              ck(h, launch_group(ctx, bt, hp, s), "libgint_replay_noalloc: k_group launch");
    };
    // The segments that fit a share of the scratch run on the worker streams, each stream in its
    // own share, as the ordinary replay does: a small system's segments are far too small to fill the
-   // GPU one after another (4 molecules, 81 classes: 3.5 ms in a row, 0.68 ms so). The others follow on the
-   // caller's stream, one after another in the whole scratch. A stream being captured keeps to itself.
+   // GPU one after another (4 molecules, 81 classes: 3.5 ms in a row, 0.4 ms so). The others follow on
+   // the caller's stream, one after another in the whole scratch. All worker streams take part where
+   // every segment fits the smaller share. A stream being captured keeps to itself.
    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
    if (!ck(h, cudaStreamIsCapturing(st, &cap), "libgint_replay_noalloc: capture status")) return h->err;
-   const size_t share = (kNoAllocScratchDoubles / kWorkStreams) & ~(size_t)31;
-   auto small = [&](const Handle::RecSeg &g) {
-      const ClassPlan &hp = h->plans[g.c & 255];
-      return cap == cudaStreamCaptureStatusNone && (((size_t)g.nprm * hp.S + 31) & ~(size_t)31) + scratch_of(hp) <= share;
+   auto size_of = [&](const Handle::RecSeg &g) {
+      return (((size_t)g.nprm * h->plans[g.c & 255].S + 31) & ~(size_t)31) + scratch_of(h, g.c);
    };
+   auto share_of = [](int n) { return (kNoAllocScratchDoubles / n) & ~(size_t)31; };
+   int workers = kWorkStreams;
+   for (auto &rb : h->recs)
+      for (auto &g : rb.segs)
+         if (size_of(g) > share_of(kWorkStreams)) workers = kFewWorkStreams;
+   const size_t share = share_of(workers);
+   auto small = [&](const Handle::RecSeg &g) { return cap == cudaStreamCaptureStatusNone && size_of(g) <= share; };
    bool ok = true;
    int n = 0;
    for (auto &rb : h->recs)
@@ -1967,14 +1992,14 @@ int libgint_replay_noalloc(void *hh, const double *P_dev, double *K_dev, size_t 
          if (!ok || !small(g)) continue;
          if (n == 0) {
             ok = ck(h, cudaEventRecord(h->fork_ev, st), "libgint_replay_noalloc: event record");
-            for (int w = 0; ok && w < kWorkStreams; w++)
+            for (int w = 0; ok && w < workers; w++)
                ok = ck(h, cudaStreamWaitEvent(h->work[w], h->fork_ev, 0), "libgint_replay_noalloc: stream wait");
             if (!ok) break;
          }
-         const int w = n++ % kWorkStreams;
+         const int w = n++ % workers;
          ok = run(rb, g, scr + (size_t)w * share, share, h->work[w]);
       }
-   for (int w = 0; n && w < kWorkStreams; w++)
+   for (int w = 0; n && w < workers; w++)
       ok = ck(h, cudaEventRecord(h->work_ev[w], h->work[w]), "libgint_replay_noalloc: event record") &&
            ck(h, cudaStreamWaitEvent(st, h->work_ev[w], 0), "libgint_replay_noalloc: stream wait") && ok;
    for (auto &rb : h->recs)
