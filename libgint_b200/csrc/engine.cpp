@@ -284,7 +284,7 @@ struct Handle {
    std::vector<SetFast> fast;
    bool basis_dirty = true, ent_dirty = true;
    // device-resident data
-   DBuf d_pool, d_ents, d_neighs, d_img, d_C0, d_C0f, d_lut, d_bw, d_ft, d_plans, d_err, d_vops, d_tmap;
+   DBuf d_pool, d_ents, d_neighs, d_img, d_order, d_C0, d_C0f, d_lut, d_bw, d_ft, d_plans, d_err, d_vops, d_tmap;
    char *stage = nullptr;           // pinned chunks of staged_copy
    cudaEvent_t stage_ev[8] = {};
    DBuf d_tmax;                     // incremental replays: tile maxima of |dP|
@@ -425,17 +425,26 @@ static bool h2d(Handle *h, void *dst, const void *src, size_t bytes, const char 
    return ck(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, h->stream), what);
 }
 
-// The image vectors in order of their length (ties in the caller's order), for the image sums of
-// the primitive kernels: each primitive quartet tests only the images up to a length. A vector of
-// undefined length counts as the shortest, so that every primitive tests it.
-static std::vector<double4> images_by_length(const std::vector<double> &neighs) {
-   std::vector<double4> v(neighs.size() / 3);
-   for (size_t i = 0; i < v.size(); i++) {
-      const double x = neighs[3 * i], y = neighs[3 * i + 1], z = neighs[3 * i + 2], n = std::sqrt(x * x + y * y + z * z);
-      v[i] = make_double4(x, y, z, std::isnan(n) ? 0.0 : n);
+// The image vectors and their lengths for the image sums of the primitive kernels (DevCtx::img and
+// img_order): each primitive quartet tests only the images up to a length, in the caller's order, so
+// that its sum runs over the passing images as over the whole list. A vector of undefined length
+// counts as the shortest, so that every primitive tests it.
+static void images_by_length(const std::vector<double> &neighs, std::vector<double4> &img, std::vector<uint8_t> &order) {
+   const size_t n = neighs.size() / 3;
+   std::vector<std::pair<double, int>> by(n);
+   for (size_t i = 0; i < n; i++) {
+      const double x = neighs[3 * i], y = neighs[3 * i + 1], z = neighs[3 * i + 2], r = std::sqrt(x * x + y * y + z * z);
+      by[i] = {std::isnan(r) ? 0.0 : r, (int)i};
    }
-   std::stable_sort(v.begin(), v.end(), [](const double4 &a, const double4 &b) { return a.w < b.w; });
-   return v;
+   std::sort(by.begin(), by.end());
+   img.resize(n);
+   order.assign(n * n, 0);
+   std::vector<uint8_t> sel;
+   for (size_t k = 0; k < n; k++) {
+      img[k] = make_double4(neighs[3 * k], neighs[3 * k + 1], neighs[3 * k + 2], by[k].first);
+      sel.insert(std::lower_bound(sel.begin(), sel.end(), (uint8_t)by[k].second), (uint8_t)by[k].second);
+      std::copy(sel.begin(), sel.end(), order.begin() + k * n);
+   }
 }
 
 // Copies a large P or K between the caller's pageable array and the device through pinned memory,
@@ -582,10 +591,13 @@ static bool upload_tables(Handle *h) {
    if (h->neighs_dirty) {
       if (!ensure(h, h->d_neighs, h->neighs.size() * 8, "neighs")) return false;
       if (!h2d(h, h->d_neighs.p, h->neighs.data(), h->neighs.size() * 8, "neighs")) return false;
-      const std::vector<double4> img = images_by_length(h->neighs);
+      std::vector<double4> img;
+      std::vector<uint8_t> order;
+      images_by_length(h->neighs, img, order);
+      if (!ensure(h, h->d_order, order.size(), "neighs") || !h2d(h, h->d_order.p, order.data(), order.size(), "neighs")) return false;
       if (!ensure(h, h->d_img, img.size() * sizeof(double4), "neighs")) return false;
       if (!h2d(h, h->d_img.p, img.data(), img.size() * sizeof(double4), "neighs")) return false;
-      // img goes out of scope: wait for its copy
+      // the sources go out of scope: wait for their copies
       if (!ck(h, cudaStreamSynchronize(h->stream), "neighs")) return false;
       h->neighs_dirty = false;
       uploaded = true;
@@ -648,6 +660,7 @@ static DevCtx make_ctx(Handle *h) {
    c.ents = (const BasisEnt *)h->d_ents.p;
    c.neighs = (const double *)h->d_neighs.p;
    c.img = (const double4 *)h->d_img.p;
+   c.img_order = (const uint8_t *)h->d_order.p;
    c.Ng = h->Ng;
    c.nspin = h->nspin;
    std::memcpy(c.cell, h->cell, sizeof(c.cell));
@@ -2153,7 +2166,7 @@ void libgint_destroy_handle(void *hh) {
    }
    for (auto &rb : h->recs) { release(rb.rec); release(rb.gbuf); }
    release(h->rec_ac); release(h->rec_gscr); release(h->d_cnt);
-   DBuf *bufs[] = {&h->d_pool, &h->d_ents, &h->d_neighs, &h->d_img, &h->d_C0, &h->d_C0f, &h->d_lut, &h->d_bw, &h->d_ft, &h->d_vops, &h->d_tmap, &h->d_tmax,
+   DBuf *bufs[] = {&h->d_pool, &h->d_ents, &h->d_neighs, &h->d_img, &h->d_order, &h->d_C0, &h->d_C0f, &h->d_lut, &h->d_bw, &h->d_ft, &h->d_vops, &h->d_tmap, &h->d_tmax,
                    &h->d_plans, &h->d_err};
    for (DBuf *b : bufs) release(*b);
    h->team.reset();

@@ -197,13 +197,13 @@ cudaError_t launch_lanes(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st
    // 32 / TPR rows per warp: rows cost from one primitive to thousands, so the block scheduler, which
    // starts a new block wherever one finishes, balances them better than a grid-stride loop
    const long blocks = std::max(1L, std::min(((long)bt.nqrtt * TPR + threads - 1) / threads, 1L << 30));
-   if constexpr (class_has_fp32(LA, LB, LC, LD)) {
-      if (bt.fp32) {
-         k_group3<LA, LB, LC, LD, float, TPR><<<(unsigned)blocks, threads, 0, st>>>(ctx, bt);
+   if (bt.fp32) {
+      if constexpr (class_has_fp32(LA, LB, LC, LD) && TPR == 1) {
+         k_group3<LA, LB, LC, LD, float, 1><<<(unsigned)blocks, threads, 0, st>>>(ctx, bt);
          return cudaGetLastError();
+      } else {
+         return cudaErrorInvalidValue;   // no FP32 segments for these classes, and none with more lanes
       }
-   } else {
-      if (bt.fp32) return cudaErrorInvalidValue;   // no FP32 segments for these classes
    }
    k_group3<LA, LB, LC, LD, double, TPR><<<(unsigned)blocks, threads, 0, st>>>(ctx, bt);
    return cudaGetLastError();
@@ -216,7 +216,8 @@ cudaError_t launch_one(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st) 
    // rows enough: the line lies where the GPU has nothing else to run.) The classes of L <= 3, kernels one
    // after another: 4 molecules l <= 2 2.70 -> 0.97 ms, 24 clusters 6.85 -> 2.93 ms, 32 molecules
    // l <= 2 2.83 -> 1.38 ms; the 1/4096 sample of 64 molecules, with 150k rows and more a class, unchanged.
-   if (bt.nqrtt < 148u * 64 * Group3Shape<LA, LB, LC, LD>::MINB) return launch_lanes<LA, LB, LC, LD, 4>(ctx, bt, st);
+   // FP32 rows keep one lane: there the order of a sum shows in K at the accuracy of the path.
+   if (!bt.fp32 && bt.nqrtt < 148u * 64 * Group3Shape<LA, LB, LC, LD>::MINB) return launch_lanes<LA, LB, LC, LD, 4>(ctx, bt, st);
    return launch_lanes<LA, LB, LC, LD, 1>(ctx, bt, st);
 }
 
@@ -251,7 +252,6 @@ struct PartPreload {
          if ((e = cudaFuncGetAttributes(&a, k_group3<la, lb, lc, ld, double, 4>)) != cudaSuccess) return e;
          if constexpr (class_has_fp32(la, lb, lc, ld)) {
             if ((e = cudaFuncGetAttributes(&a, k_group3<la, lb, lc, ld, float, 1>)) != cudaSuccess) return e;
-            if ((e = cudaFuncGetAttributes(&a, k_group3<la, lb, lc, ld, float, 4>)) != cudaSuccess) return e;
          }
          return PartPreload<I + kGroup3Parts>::run();
       }

@@ -113,7 +113,8 @@ k_prim2(DevCtx ctx, BatchArgs bt, int cp, int team_doubles) {
       }
       tsync<NT>();
       int start;
-      const int npair = pair_starts(lane < np ? image_count(ctx.img, Ng, geo[lane]) : 0, np, lane, start);
+      const int nimg = lane < np ? image_count(ctx.img, Ng, geo[lane]) : 0;
+      const int npair = pair_starts(nimg, np, lane, start);
       double *out = bt.AC + (size_t)p0 * S;
       unsigned done = 0;   // primitives whose row holds an image already
       // stages 3 and 4 of the queued pairs [0, cnt)
@@ -180,7 +181,7 @@ k_prim2(DevCtx ctx, BatchArgs bt, int cp, int team_doubles) {
          bool pass = false;
          double T = 0.0;
          int tn;
-         const int tp = pair_prim(b0, start, lane, tn);
+         const int tp = pair_prim(ctx, b0, npair, start, nimg, lane, tn);
          if (b0 + lane < npair) {
             const PrimGeo &g = geo[tp];
             const double *im = reinterpret_cast<const double *>(ctx.img + tn);

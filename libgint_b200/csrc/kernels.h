@@ -17,7 +17,8 @@ struct DevCtx {
    const double *pool;        // exponents and normalised coefficients
    const BasisEnt *ents;
    const double *neighs;      // Ng lattice vectors
-   const double4 *img;        // the same in order of their length: {vector, length}
+   const double4 *img;        // {lattice vector i, i-th smallest length of a lattice vector}
+   const uint8_t *img_order;  // [Ng][Ng]: row n - 1 holds the n shortest vectors' indices, ascending
    int Ng;
    int nspin;
    double cell[18];           // h (rows = lattice vectors) and h^-1

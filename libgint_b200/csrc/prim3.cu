@@ -65,7 +65,7 @@ k_prim3(DevCtx ctx, BatchArgs bt, int cp) {
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = blockDim.x >> 5;
    const int Ng = ctx.Ng;
    write_shell_vectors(ctx, bt);
-   // the image vectors in order of length, shared by the block
+   // the image vectors and lengths, shared by the block
    double4 *simg = reinterpret_cast<double4 *>(smem);
    for (int i = threadIdx.x; i < 4 * Ng; i += blockDim.x) smem[i] = __ldg(reinterpret_cast<const double *>(ctx.img) + i);
    __syncthreads();
@@ -182,7 +182,7 @@ k_prim3(DevCtx ctx, BatchArgs bt, int cp) {
          bool pass = false;
          double T = 0.0;
          int tn;
-         const int tp = pair_prim(b0, start, lane, tn);
+         const int tp = pair_prim(ctx, b0, npair, start, nimg, lane, tn);
          if (b0 + lane < npair) {
             const PrimGeo &g = geo[tp];
             const double4 im = simg[tn];
@@ -247,7 +247,8 @@ cudaError_t launch_one(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st) 
    // fills a G_m batch (one pair each without images, about four each with them) unless it is too
    // small for one such chunk an SM; and it is spread over the SMs before a block takes more warps.
    const long slots = 148L * Sh::MINB * nwmax;
-   const int cpmin = ctx.Ng == 1 ? Sh::CP : std::min(bt.nprm < 148u * 8 ? 2 : 8, Sh::CP);
+   // (The FP32 path keeps CP: where a chunk's batches end decides how its image sums round.)
+   const int cpmin = ctx.Ng == 1 || sizeof(R) == 4 ? Sh::CP : std::min(bt.nprm < 148u * 8 ? 2 : 8, Sh::CP);
    const int cp = (int)std::max((long)cpmin, std::min((long)Sh::CP, ((long)bt.nprm + slots - 1) / slots));
    const long nchunk = ((long)bt.nprm + cp - 1) / cp;
    const int nw = (int)std::max(1L, std::min((long)nwmax, (nchunk + 147) / 148));

@@ -198,7 +198,7 @@ static __device__ __forceinline__ void kill_if_screened(const BatchArgs &bt, con
    if (bt.gflags && !__ldg(bt.gflags + sh.group)) g.upper = -1.0;
 }
 
-// How many of the images, in order of their length, can pass the truncation test of a primitive:
+// How many of the images, shortest first, can pass the truncation test of a primitive:
 // rho |D - g|^2 <= upper needs |g| <= |D| + sqrt(upper / rho). The bound is widened by far more than
 // the test's rounding, so it leaves out only images that the test refuses; at least one is kept, so
 // that every primitive has a place in the pair numbering. (An undefined bound keeps all.) With 125
@@ -230,13 +230,17 @@ static __device__ __forceinline__ int pair_starts(int n, int np, int lane, int &
    return __shfl_sync(0xffffffffu, sum, 31);
 }
 
-// The primitive of pair b0 + lane, and its image's number among the primitive's.
-static __device__ __forceinline__ int pair_prim(int b0, int start, int lane, int &n3) {
+// The primitive of pair b0 + lane of npair and its image, the n-th of the primitive's `count` shortest in
+// the caller's order (undefined beyond the last pair).
+static __device__ __forceinline__ int pair_prim(const DevCtx &ctx, int b0, int npair, int start, int count, int lane,
+                                                int &n3) {
    const unsigned rel = (unsigned)start - (unsigned)b0;
    const unsigned starts = __reduce_or_sync(0xffffffffu, start >= b0 && rel < 32u ? 1u << rel : 0u);
    const int before = __popc(__ballot_sync(0xffffffffu, start < b0));
    const int p = before + __popc(starts & ((2u << lane) - 1u)) - 1;
-   n3 = b0 + lane - __shfl_sync(0xffffffffu, start, p);
+   const int n = b0 + lane - __shfl_sync(0xffffffffu, start, p);
+   const int row = __shfl_sync(0xffffffffu, count, p) - 1;
+   n3 = b0 + lane < npair ? __ldg(ctx.img_order + row * ctx.Ng + n) : 0;
    return p;
 }
 
