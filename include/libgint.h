@@ -164,7 +164,7 @@ double libgint_replay_profile_classes(void *handle, double *kt, double *kcls);
  * libgint_autotune times, for every class of the recorded quartet list, the primitive kernel with
  * generated per-lane VRR against the per-warp interpreted one, and the group kernel with one lane
  * per contraction row (generated HRR; classes with la+lb+lc+ld <= 3) or one block per set quartet
- * (the HRR and spherical transform as dense products; the other classes) against one warp per row
+ * (contraction on the tensor cores, HRR in registers; the other classes) against one warp per row
  * (interpreted HRR), and keeps the faster of each for every following launch;
  * out[2c], out[2c+1] (c = la*64+lb*16+lc*4+ld; 512 ints, may be NULL) receive the choices
  * (0 = per-lane or per-block, 1 = per-warp). libgint_set_tuning installs such a table,

@@ -17,7 +17,7 @@ HOSTCXX = "g++"
 # generated classes compile in parallel
 PRIM3_PARTS = 8
 GROUP3_PARTS = 4
-GROUP_MM_PARTS = 4
+GROUP_MM_PARTS = 11
 # engine.cpp holds the team-collective calls (orphaned OpenMP constructs bound to the caller's team)
 ENGINE_OBJS = [("engine.cpp", ["-Xcompiler", "-fopenmp"], "engine.o"), ("plan.cpp", [], "plan.o"), ("kernels.cu", [], "kernels.o")] + \
     [("prim3.cu", [f"-DPRIM3_PART={i}"], f"prim3_{i}.o") for i in range(PRIM3_PARTS)] + \

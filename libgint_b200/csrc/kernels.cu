@@ -240,17 +240,6 @@ k_prim2(DevCtx ctx, BatchArgs bt, int cp, int team_doubles) {
 // One group (all image pairs of one set quartet, all contraction rows) processed by NL
 // cooperating lanes (NL = 32: one warp; NL = 1: one lane) whose workspace element x lives at
 // ws[x * ST] (ST = 32 for lane-interleaved per-lane workspaces).
-// Nonzero pattern of the cartesian -> spherical rows (bit k of kC2sMask[l][m]: coefficient k of
-// row m), the integer solid-harmonic rows the coefficients are made from. Terms outside it are
-// exact zeros, so leaving them out changes no sum; upload_constant_tables checks the pattern
-// against the coefficients it uploads.
-__host__ __device__ constexpr uint16_t c2s_mask(int l, int m) {
-   constexpr uint16_t t[4][7] = {{0x1, 0, 0, 0, 0, 0, 0},
-                                 {0x2, 0x4, 0x1, 0, 0, 0, 0},
-                                 {0x02, 0x10, 0x29, 0x04, 0x09, 0, 0},
-                                 {0x042, 0x010, 0x142, 0x284, 0x029, 0x084, 0x009}};
-   return t[l][m];
-}
 
 // One spherical pass over centre LX: the workspace is [npre][ncart(LX)][npost] in, and
 // [npre][2LX+1][npost] out. Each lane transforms whole vectors (one (pre, post) pair at a time),
@@ -700,7 +689,7 @@ size_t group_global_scratch(const ClassPlan &hp, int *grid, int *warps) {
 
 
 // Group-kernel choice on variant 0: k_group3 (generated HRR, one lane per row) for the classes it
-// covers, k_group_mm (dense products, one block per group) for the others; on variant 1 always
+// covers, k_group_mm (one block per group) for the others; on variant 1 always
 // k_group (one warp per row).
 cudaError_t launch_group(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan &hp, cudaStream_t st) {
    if (bt.nqrtt == 0) return cudaSuccess;
@@ -709,7 +698,7 @@ cudaError_t launch_group(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan
       if (group3_launch(ctx, bt, st, &err)) return err;
    }
    if (bt.fp32) return cudaErrorInvalidValue;   // FP32 segments exist only for classes with k_group3
-   if (bt.group_variant == 0) return group_mm_launch(ctx, bt, hp, max_dyn_smem(), st);
+   if (bt.group_variant == 0) return group_mm_launch(ctx, bt, st);
    const size_t wd = group_warp_doubles(hp);
    const size_t plan_bytes = group_hdr_bytes();
    const int nw = group_smem_warps(wd);

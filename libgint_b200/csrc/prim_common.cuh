@@ -430,6 +430,18 @@ static __device__ __forceinline__ SegSum<R> make_segsum(int key, int lane, R *ds
    return sg;
 }
 
+// Nonzero pattern of the cartesian -> spherical rows (bit k of kC2sMask[l][m]: coefficient k of
+// row m), the integer solid-harmonic rows the coefficients are made from. Terms outside it are
+// exact zeros, so leaving them out changes no sum; upload_constant_tables checks the pattern
+// against the coefficients it uploads.
+__host__ __device__ constexpr uint16_t c2s_mask(int l, int m) {
+   constexpr uint16_t t[4][7] = {{0x1, 0, 0, 0, 0, 0, 0},
+                                 {0x2, 0x4, 0x1, 0, 0, 0, 0},
+                                 {0x02, 0x10, 0x29, 0x04, 0x09, 0, 0},
+                                 {0x042, 0x010, 0x142, 0x284, 0x029, 0x084, 0x009}};
+   return t[l][m];
+}
+
 // whether the four P/K blocks that a row reads and updates lie inside the arrays
 static __device__ __forceinline__ bool row_in_range(const QrttRec &k, int na, int nb, int nc, int nd, size_t n) {
    const int nx[4] = {na, na, nb, nb}, ny[4] = {nc, nd, nc, nd};
