@@ -120,10 +120,9 @@ struct Group3Shape {
 
 // R = double: the FP64 path; R = float: the FP32 path (contraction, HRR and spherical transform in
 // FP32 from the FP32 targets of k_prim3; the K update in FP64).
-// TPR lanes share one contraction row: they divide its primitives, add their targets up, and all go on
-// with the sums.
+// TPR lanes share one contraction row: they divide its targets, and all go on with all of them.
 template <int LA, int LB, int LC, int LD, class R, int TPR>
-__global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB) k_group3(DevCtx ctx, BatchArgs bt) {
+__global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB / (TPR == 1 ? 1 : 2)) k_group3(DevCtx ctx, BatchArgs bt) {
    using G = GrpGen<LA, LB, LC, LD>;
    constexpr int S = G::S, Nc = G::Nc, Ns = G::Ns;
    const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
@@ -156,22 +155,54 @@ __global__ void __launch_bounds__(128, Group3Shape<LA, LB, LC, LD>::MINB) k_grou
          R T[S];
 #pragma unroll
          for (int j = 0; j < S; j++) T[j] = R(0);
-         const R *AC = reinterpret_cast<const R *>(bt.AC);
-         // contraction over the primitives (reference src/compute_ECO.cpp:131-212); four per
-         // iteration so that the next ones' loads overlap this one's FMAs
-#pragma unroll 4
-         for (uint32_t ip = sub; ip < sh.nprm; ip += TPR) {
+         // contraction over the primitives (reference src/compute_ECO.cpp:131-212)
+         const R *ac = reinterpret_cast<const R *>(bt.AC) + (size_t)sh.prm_off * S;
+         auto coef = [&](uint32_t ip) {
             const uint32_t code = __ldg(bt.prm + sh.prm_off + ip);
-            const R kp = (R)__ldg(Ka + (code >> 24)) * (R)__ldg(Kb + ((code >> 16) & 255)) *
-                         (R)__ldg(Kc + ((code >> 8) & 255)) * (R)__ldg(Kd + (code & 255));
-            const R *row = AC + (size_t)(sh.prm_off + ip) * S;
+            return (R)__ldg(Ka + (code >> 24)) * (R)__ldg(Kb + ((code >> 16) & 255)) * (R)__ldg(Kc + ((code >> 8) & 255)) *
+                   (R)__ldg(Kd + (code & 255));
+         };
+         if constexpr (TPR == 1) {
+            // four per iteration so that the next ones' loads overlap this one's FMAs
+#pragma unroll 4
+            for (uint32_t ip = 0; ip < sh.nprm; ip++) {
+               const R kp = coef(ip);
+               const R *row = ac + (size_t)ip * S;
 #pragma unroll
-            for (int j = 0; j < S; j++) T[j] += kp * __ldg(row + j);
+               for (int j = 0; j < S; j++) T[j] += kp * __ldg(row + j);
+            }
+         } else {
+            // lane `sub` sums targets sub, sub + TPR, ... over the primitives in their order, and makes the
+            // coefficient of every TPR-th primitive; the loads of TPR * UP primitives are under way at a time
+            constexpr int SQ = (S + TPR - 1) / TPR, UP = SQ <= 2 ? 4 : (SQ <= 4 ? 2 : 1);
+            R t[SQ];
+#pragma unroll
+            for (int i = 0; i < SQ; i++) t[i] = R(0);
+            for (uint32_t p0 = 0; p0 < sh.nprm; p0 += TPR * UP) {
+               R mine[UP], a[UP][TPR][SQ];
+#pragma unroll
+               for (int u = 0; u < UP; u++) {
+                  mine[u] = p0 + u * TPR + sub < sh.nprm ? coef(p0 + u * TPR + sub) : R(0);
+#pragma unroll
+                  for (int k = 0; k < TPR; k++)
+#pragma unroll
+                     for (int i = 0; i < SQ; i++) {
+                        const uint32_t ip = p0 + u * TPR + k;
+                        a[u][k][i] = ip < sh.nprm && i * TPR + sub < S ? __ldg(ac + (size_t)ip * S + i * TPR + sub) : R(0);
+                     }
+               }
+#pragma unroll
+               for (int u = 0; u < UP; u++)
+#pragma unroll
+                  for (int k = 0; k < TPR; k++) {
+                     const R kp = __shfl_sync(team, mine[u], lane - sub + k);
+#pragma unroll
+                     for (int i = 0; i < SQ; i++) t[i] += kp * a[u][k][i];
+                  }
+            }
+#pragma unroll
+            for (int j = 0; j < S; j++) T[j] = __shfl_sync(team, t[j / TPR], lane - sub + j % TPR);
          }
-#pragma unroll
-         for (int o = 1; o < TPR; o <<= 1)
-#pragma unroll
-            for (int j = 0; j < S; j++) T[j] += __shfl_xor_sync(team, T[j], o);
          double v[6];
          read_shell_vectors(ctx, bt, Gr.shell_off + s, sh, v);
          const R AB[3] = {(R)v[0], (R)v[1], (R)v[2]}, CD[3] = {(R)v[3], (R)v[4], (R)v[5]};
@@ -214,9 +245,10 @@ cudaError_t launch_one(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st) 
    // Too few rows to fill half of the warps that the registers leave room for: four lanes a row. (The
    // rows of one set quartet read the same targets, so more lanes a row cost reads where there are
    // rows enough: the line lies where the GPU has nothing else to run.) The classes of L <= 3, kernels one
-   // after another: 4 molecules l <= 2 2.70 -> 0.97 ms, 24 clusters 6.85 -> 2.93 ms, 32 molecules
-   // l <= 2 2.83 -> 1.38 ms; the 1/4096 sample of 64 molecules, with 150k rows and more a class, unchanged.
-   // FP32 rows keep one lane: there the order of a sum shows in K at the accuracy of the path.
+   // after another: 4 molecules l <= 2 2.70 -> 0.69 ms, 24 clusters 6.85 -> 2.40 ms, 32 molecules
+   // l <= 2 2.83 -> 1.04 ms; the 1/4096 sample of 64 molecules, with 150k rows and more a class, unchanged.
+   // (Lanes that divided the primitives took 1.03, 2.90 and 1.36 ms, and changed the order of their sum.)
+   // FP32 rows keep one lane: few segments of theirs are that small.
    if (!bt.fp32 && bt.nqrtt < 148u * 64 * Group3Shape<LA, LB, LC, LD>::MINB) return launch_lanes<LA, LB, LC, LD, 4>(ctx, bt, st);
    return launch_lanes<LA, LB, LC, LD, 1>(ctx, bt, st);
 }
