@@ -185,8 +185,10 @@ int libgint_plan_flops(int la, int lb, int lc, int ld, double *out);
  * use a fixed 64 MiB device scratch array inside the library, held by every GPU that loads it
  * until exit; each recorded class segment must fit it (record with a small
  * libgint_set_max_mem, e.g. 150), otherwise the call fails with a clear error. K_dev is zeroed
- * first. The first call on a device looks up the scratch address (make it before any stream
- * capture); calls that overlap on the GPU share the scratch and race. Returns 0 or the error. */
+ * first. Small segments run on the handle's own streams, which wait for `stream` and which `stream`
+ * then waits for. A stream that is being captured is refused (the recording's uploads, which the call
+ * waits for, are outside the capture) and its capture goes on; calls that overlap on the GPU share the
+ * scratch and race. Returns 0 or the error. */
 int libgint_replay_noalloc(void *handle, const double *P_dev, double *K_dev, size_t K_size, void *stream);
 /* per-class device event counters: out[c*4 + {0,1,2,3}] = Chebyshev G_m evaluations, Boys
  * evaluations, images through the VRR, primitive quartets; c = la*64 + lb*16 + lc*4 + ld */

@@ -1922,6 +1922,15 @@ int libgint_replay_noalloc(void *hh, const double *P_dev, double *K_dev, size_t 
    // the handle's device holds the recording, the plans and the scratch this call uses
    use_device(h);
    if (h->err) return h->err;
+   cudaStream_t st = stream ? (cudaStream_t)stream : h->stream;
+   // The call orders its stream after the recording's uploads, which lie outside any capture, so it
+   // cannot be captured. Refused before it adds anything, which leaves the caller's capture valid.
+   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+   if (!ck(h, cudaStreamIsCapturing(st, &cap), "libgint_replay_noalloc: capture status")) return h->err;
+   if (cap != cudaStreamCaptureStatusNone) {
+      ck(h, cudaErrorStreamCaptureIsolation, "libgint_replay_noalloc: the stream is being captured");
+      return h->err;
+   }
    double *scr = nullptr;
    if (!ck(h, noalloc_scratch(&scr), "libgint_replay_noalloc: scratch lookup")) return h->err;
    // every class segment must fit: image-summed targets [nprm][S], then the HRR workspace
@@ -1941,7 +1950,6 @@ int libgint_replay_noalloc(void *hh, const double *P_dev, double *K_dev, size_t 
          }
       }
    }
-   cudaStream_t st = stream ? (cudaStream_t)stream : h->stream;
    // the recorded batches' uploads (queued on the handle's stream by the recording build) come first
    if (st != h->stream) {
       if (!ck(h, cudaEventRecord(h->noalloc_ev, h->stream), "libgint_replay_noalloc: event record") ||
@@ -1985,9 +1993,7 @@ int libgint_replay_noalloc(void *hh, const double *P_dev, double *K_dev, size_t 
    // own share, as the ordinary replay does: a small system's segments are far too small to fill the
    // GPU one after another (4 molecules, 81 classes: 3.5 ms in a row, 0.4 ms so). The others follow on
    // the caller's stream, one after another in the whole scratch. All worker streams take part where
-   // every segment fits the smaller share. A stream being captured keeps to itself.
-   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-   if (!ck(h, cudaStreamIsCapturing(st, &cap), "libgint_replay_noalloc: capture status")) return h->err;
+   // every segment fits the smaller share.
    auto size_of = [&](const Handle::RecSeg &g) {
       return (((size_t)g.nprm * h->plans[g.c & 255].S + 31) & ~(size_t)31) + scratch_of(h, g.c);
    };
@@ -1997,7 +2003,7 @@ int libgint_replay_noalloc(void *hh, const double *P_dev, double *K_dev, size_t 
       for (auto &g : rb.segs)
          if (size_of(g) > share_of(kWorkStreams)) workers = kFewWorkStreams;
    const size_t share = share_of(workers);
-   auto small = [&](const Handle::RecSeg &g) { return cap == cudaStreamCaptureStatusNone && size_of(g) <= share; };
+   auto small = [&](const Handle::RecSeg &g) { return size_of(g) <= share; };
    bool ok = true;
    int n = 0;
    for (auto &rb : h->recs)

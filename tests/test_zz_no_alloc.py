@@ -138,3 +138,31 @@ def test_replay_noalloc_rejects_missing_recording(engine_so):
     code, msg = g.last_error()
     assert rc != 0 and code != 0 and "libgint_record" in msg
     g.close()
+
+
+@pytest.mark.gpu
+def test_replay_noalloc_refuses_a_capturing_stream_and_leaves_its_capture(engine_so):
+    import torch
+    from libgint_b200.capi import load_engine
+    torch.cuda.set_device(0)
+    lib = load_engine()
+    wl = Workload("small_l2", setq_stride=50)
+    s = Session(Api(engine_so), wl, max_mem_mb=150)
+    h = ctypes.c_void_p(s.h)
+    lib.libgint_record(h, 1)
+    s.build_K()
+    lib.libgint_record(h, 0)
+    P_dev = torch.from_numpy(wl.Pflat).cuda()
+    K_dev = torch.full((wl.Pflat.size,), 3.0, dtype=torch.float64, device="cuda")
+    x, y = torch.ones(8, device="cuda"), torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        rc = lib.libgint_replay_noalloc(h, ctypes.c_void_p(P_dev.data_ptr()), ctypes.c_void_p(K_dev.data_ptr()),
+                                        wl.Pflat.size, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        y.add_(x)
+    assert rc != 0 and b"captured" in lib.libgint_error_string(h)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((y == 1.0).all()) and bool((K_dev == 3.0).all())
+    s.close()
