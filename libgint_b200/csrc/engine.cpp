@@ -325,6 +325,7 @@ struct Handle {
    bool merge_rec = false;          // libgint_record(h, 2): one segment per queue class at the end
    std::vector<RecBatch> recs;
    long long rec_gen = 0;           // bumped whenever the recording changes
+   long long few_streams_gen = -1;  // the recording whose replay found no room for all streams' arenas
    // the replay captured as a CUDA graph, and what it was captured with
    struct GraphKey { DevCtx ctx; long long rec_gen; void *ac, *gscr; size_t half; double eps; int streams; };
    cudaGraphExec_t graph_exec = nullptr;
@@ -1047,7 +1048,21 @@ static bool prepare_replay(Handle *h, size_t *half, bool all_scratch = false) {
       }
    const size_t few = arenas(kFewWorkStreams), all = arenas(kWorkStreams);
    h->replay_streams = many_streams(prims, segs) && all <= std::max(few, h->max_mem_mb * (size_t)(1 << 20) / 64)
+                                   && h->few_streams_gen != h->rec_gen
                            ? kWorkStreams : kFewWorkStreams;
+   // where the device has no room for the arenas of all streams, the few streams' must do (and the
+   // larger buffer is not asked for again for this recording)
+   if (h->replay_streams == kWorkStreams && all > few && h->rec_ac.bytes < all * 8) {
+      release(h->rec_ac);
+      if (cudaMalloc(&h->rec_ac.p, all * 8) == cudaSuccess) {
+         h->rec_ac.bytes = all * 8;
+      } else {
+         cudaGetLastError();
+         h->rec_ac.p = nullptr;
+         h->few_streams_gen = h->rec_gen;
+         h->replay_streams = kFewWorkStreams;
+      }
+   }
    ac = h->replay_streams == kWorkStreams ? all : arenas(kFewWorkStreams);
    if (!ensure(h, h->rec_ac, std::max<size_t>(ac * 8, 256), "replay AC")) return false;
    if (gs && !ensure(h, h->rec_gscr, gs * 8, "replay HRR scratch")) return false;
