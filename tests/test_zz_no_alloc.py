@@ -101,6 +101,37 @@ def test_replay_noalloc_right_after_recording_multi_batch_periodic(engine_so, or
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("variant", [0, 1])
+def test_replay_noalloc_without_room_for_the_displacements(engine_so, variant):
+    """Three primitives to an (ss|ss) shell quartet, whose displacements take twice the room of its targets:
+    the segment fits its share of the scratch (a sixth of 64 MiB), the displacements do not, and the group
+    kernel (either choice) derives them itself."""
+    import torch
+    from libgint_b200.capi import load_engine
+    torch.cuda.set_device(0)
+    lib = load_engine()
+    wl = Workload("periodic_l2_small", setq_stride=8)
+    ls = wl.sets()[:, 1][wl.setq()[:, :4]]
+    nshell, nprim = wl.setq()[ls.sum(axis=1) == 0][:, 4:6].sum(axis=0)
+    share = 8 * 1024 * 1024 // 6
+    assert nprim <= share < nprim + 6 * nshell
+    s = Session(Api(engine_so), wl, max_mem_mb=7000)
+    h = ctypes.c_void_p(s.h)
+    lib.libgint_record(h, 2)
+    s.build_K()
+    lib.libgint_record(h, 0)
+    tune = (ctypes.c_int * 512)()
+    tune[1] = variant
+    lib.libgint_set_tuning(h, tune)
+    P, K = wl.Pflat, np.zeros(wl.Pflat.size)
+    lib.libgint_set_P(h, P.ctypes.data_as(D), P.size)
+    assert lib.libgint_replay(h) > 0
+    lib.libgint_get_K(h, K.ctypes.data_as(D))
+    _noalloc_twice(lib, h, P, K, K)
+    s.close()
+
+
+@pytest.mark.gpu
 def test_replay_noalloc_rejects_a_segment_beyond_the_scratch(engine_so):
     """A recording made with a large work budget holds class segments larger than the fixed
     scratch: the call fails with error 5 before launching anything, and the caller's K is left
