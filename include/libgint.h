@@ -122,7 +122,8 @@ const char *libgint_error_string(void *handle);
 void libgint_destroy_handle(void *handle);
 /* sizes of the recursion plan of class (la,lb,lc,ld): out[0..7] = VRR workspace, contracted
  * targets, HRR workspace (doubles), cartesian and spherical block sizes, VRR blocks, HRR
- * steps, primitive team size; returns 0 for an unsupported class */
+ * steps, threads that the interpreted primitive kernel gives one primitive's VRR in a segment that fills
+ * the GPU; returns 0 for an unsupported class */
 int libgint_plan_sizes(int la, int lb, int lc, int ld, int *out);
 /* the HRR instructions of class (la,lb,lc,ld) as the interpreted group kernel runs them: out[2i],
  * out[2i+1] = {in1 | axis << 30, in2} computing workspace element S + i as

@@ -1246,8 +1246,8 @@ static void record_group_pmax(Handle *h) {
 }
 
 // The autotuner: for every class of the recording, the primitive kernels (generated per-lane VRR,
-// variant 0, against the per-warp interpreted VRR, variant 1) and the group kernels (one lane per
-// contraction row with generated HRR, variant 0, against one warp per row with the interpreted HRR,
+// variant 0, against the interpreted VRR, variant 1) and the group kernels (one lane per contraction
+// row, or one block per set quartet, variant 0, against one warp per row with the interpreted HRR,
 // variant 1) are timed on the class's recorded segments, serialised on the handle's stream with
 // CUDA events, and the faster of each is kept. FP32 segments have only variant 0. K is zeroed
 // afterwards (the timing runs add into it).

@@ -248,7 +248,7 @@ cudaError_t launch_one(const DevCtx &ctx, const BatchArgs &bt, cudaStream_t st) 
    // after another: 4 molecules l <= 2 2.70 -> 0.69 ms, 24 clusters 6.85 -> 2.40 ms, 32 molecules
    // l <= 2 2.83 -> 1.04 ms; the 1/4096 sample of 64 molecules, with 150k rows and more a class, unchanged.
    // (Lanes that divided the primitives took 1.03, 2.90 and 1.36 ms, and changed the order of their sum.)
-   // FP32 rows keep one lane: few segments of theirs are that small.
+   // FP32 rows keep one lane: there is no FP32 instance of four.
    if (!bt.fp32 && bt.nqrtt < 148u * 64 * Group3Shape<LA, LB, LC, LD>::MINB) return launch_lanes<LA, LB, LC, LD, 4>(ctx, bt, st);
    return launch_lanes<LA, LB, LC, LD, 1>(ctx, bt, st);
 }

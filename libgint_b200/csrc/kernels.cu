@@ -237,44 +237,33 @@ k_prim2(DevCtx ctx, BatchArgs bt, int cp, int team_doubles) {
 // ---------------------------------------------------------------------------------------
 // k_group: contraction + HRR + sum over image pairs + spherical transform + K update
 // ---------------------------------------------------------------------------------------
-// One group (all image pairs of one set quartet, all contraction rows) processed by NL
-// cooperating lanes (NL = 32: one warp; NL = 1: one lane) whose workspace element x lives at
-// ws[x * ST] (ST = 32 for lane-interleaved per-lane workspaces).
-
 // One spherical pass over centre LX: the workspace is [npre][ncart(LX)][npost] in, and
 // [npre][2LX+1][npost] out. Each lane transforms whole vectors (one (pre, post) pair at a time),
 // so the coefficients are uniform across the warp. Same sum order as a dense row loop.
-template <int LX, int NL, int ST>
+template <int LX>
 static __device__ __forceinline__ void sph_pass(const double *src, double *dst, int npre, int npost, int lane) {
    constexpr int NK = (LX + 1) * (LX + 2) / 2, NSX = 2 * LX + 1;
    const int nu = npre * npost;
-   for (int u = lane; u < nu; u += NL) {
+   for (int u = lane; u < nu; u += 32) {
       const int pre = u / npost, post = u - pre * npost;
-      const double *s = src + (pre * NK * npost + post) * ST;
-      double *d = dst + (pre * NSX * npost + post) * ST;
+      const double *s = src + pre * NK * npost + post;
+      double *d = dst + pre * NSX * npost + post;
       double x[NK];
 #pragma unroll
-      for (int k = 0; k < NK; k++) x[k] = s[k * npost * ST];
+      for (int k = 0; k < NK; k++) x[k] = s[k * npost];
 #pragma unroll
       for (int m = 0; m < NSX; m++) {
          double acc = 0.0;
 #pragma unroll
          for (int k = 0; k < NK; k++)
             if (c2s_mask(LX, m) >> k & 1) acc += c_c2s[LX][m * NK + k] * x[k];
-         d[m * npost * ST] = acc;
+         d[m * npost] = acc;
       }
    }
 }
 
 // q = t / n for t * n < 2^20, with M = 2^20 / n + 1 (all spherical indices here: t < 7^4, n <= 7^3)
 static __device__ __forceinline__ int div_small(int t, uint32_t M) { return (int)(((uint32_t)t * M) >> 20); }
-
-// Synchronises the NL threads that share one row's workspace: a block (NL > 32), a warp, or none.
-template <int NL>
-static __device__ __forceinline__ void gsync() {
-   if constexpr (NL > 32) __syncthreads();
-   else if constexpr (NL > 1) __syncwarp();
-}
 
 // What the rows of one set quartet share for one shell quartet: its primitive range, the
 // coefficient rows of its four basis entries and the HRR displacements AB = A - B, CD = C - D.
@@ -298,15 +287,12 @@ static __device__ __forceinline__ void shell_shared(const DevCtx &ctx, const Bat
    for (int c = 0; c < 3; c++) { o.AB[c] = v[c]; o.CD[c] = v[3 + c]; }
 }
 
-// One contraction row q (of group gi = G) processed by NL cooperating threads (a block, a warp or
-// one lane; `lane` is the thread's index among them). With a cache slot (one warp's shared memory,
-// key ~0u at first), shell 0's shared data is derived once and reused by the next rows of the
-// same group that this warp takes.
-template <int NL, int ST>
+// One contraction row q (of group gi = G) processed by one warp with workspace ws. In the cache slot
+// (the warp's shared memory, key ~0u at first) shell 0's shared data is derived once and reused by the
+// next rows of the same group that this warp takes.
 static __device__ __forceinline__ void group_body(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan *pl,
                                                   const GroupRec &G, uint32_t q, double *ws, double *cart, int lane,
-                                                  const uint2 *hrec, double *kpw, ShellShared *cache = nullptr,
-                                                  uint32_t gi = 0) {
+                                                  const uint2 *hrec, double *kpw, ShellShared *cache, uint32_t gi) {
    const int S = pl->S, Nc = pl->Nc, Ns = pl->Ns;
    const int la = pl->la, lb = pl->lb, lc = pl->lc, ld = pl->ld;
    const int nca = ncart(la), ncb = ncart(lb), ncc = ncart(lc), ncd_ = ncart(ld);
@@ -315,17 +301,17 @@ static __device__ __forceinline__ void group_body(const DevCtx &ctx, const Batch
    {
       const int r = (int)(q - G.qrtt_off);
       const int ia = r / (nl1 * nl2 * nl3), ib = (r / (nl2 * nl3)) % nl1, ic = (r / nl3) % nl2, id = r % nl3;
-      for (int x = lane; x < Nc; x += NL) cart[x * ST] = 0.0;
+      for (int x = lane; x < Nc; x += 32) cart[x] = 0.0;
       for (uint32_t s = 0; s < G.nshell; s++) {
          ShellShared sh;
-         if (cache && s == 0 && cache->key == gi) {
+         if (s == 0 && cache->key == gi) {
             sh = *cache;
          } else {
             shell_shared(ctx, bt, G.shell_off + s, sh);
-            if (cache && s == 0) {
-               gsync<NL>();
+            if (s == 0) {
+               __syncwarp();
                if (lane == 0) { *cache = sh; cache->key = gi; }
-               gsync<NL>();
+               __syncwarp();
             }
          }
          const double *Ka = ctx.pool + sh.k_off[0] + ia * sh.np[0];
@@ -333,50 +319,37 @@ static __device__ __forceinline__ void group_body(const DevCtx &ctx, const Batch
          const double *Kc = ctx.pool + sh.k_off[2] + ic * sh.np[2];
          const double *Kd = ctx.pool + sh.k_off[3] + id * sh.np[3];
          // contraction over primitives (reference src/compute_ECO.cpp:131-212)
-         if constexpr (NL >= 32) {
-            // the contraction coefficients of 32 primitives at a time, one per thread, then every
-            // thread sums its targets over them in primitive order
-            if (sh.nprm == 0)
-               for (int j = lane; j < S; j += NL) ws[j] = 0.0;
-            for (uint32_t p0 = 0; p0 < sh.nprm; p0 += 32) {
-               const int np = (int)min(32u, sh.nprm - p0);
-               if (lane < np) {
-                  const uint32_t code = __ldg(bt.prm + sh.prm_off + p0 + lane);
-                  kpw[lane] = __ldg(Ka + (code >> 24)) * __ldg(Kb + ((code >> 16) & 255)) *
-                              __ldg(Kc + ((code >> 8) & 255)) * __ldg(Kd + (code & 255));
-               }
-               gsync<NL>();
-               const double *acp = bt.AC + (size_t)(sh.prm_off + p0) * S;
-               for (int j = lane; j < S; j += NL) {
-                  double a = p0 ? ws[j] : 0.0;
-                  const double *rp = acp + j;
-                  int q = 0;
-                  for (; q + 4 <= np; q += 4) {
-                     const double v0 = __ldg(rp), v1 = __ldg(rp + S), v2 = __ldg(rp + 2 * S), v3 = __ldg(rp + 3 * S);
-                     a += kpw[q] * v0;
-                     a += kpw[q + 1] * v1;
-                     a += kpw[q + 2] * v2;
-                     a += kpw[q + 3] * v3;
-                     rp += 4 * S;
-                  }
-                  for (; q < np; q++) { a += kpw[q] * __ldg(rp); rp += S; }
-                  ws[j] = a;
-               }
-               gsync<NL>();
+         // the contraction coefficients of 32 primitives at a time, one per lane, then every
+         // lane sums its targets over them in primitive order
+         if (sh.nprm == 0)
+            for (int j = lane; j < S; j += 32) ws[j] = 0.0;
+         for (uint32_t p0 = 0; p0 < sh.nprm; p0 += 32) {
+            const int np = (int)min(32u, sh.nprm - p0);
+            if (lane < np) {
+               const uint32_t code = __ldg(bt.prm + sh.prm_off + p0 + lane);
+               kpw[lane] = __ldg(Ka + (code >> 24)) * __ldg(Kb + ((code >> 16) & 255)) *
+                           __ldg(Kc + ((code >> 8) & 255)) * __ldg(Kd + (code & 255));
             }
-         } else {
-            for (int j = lane; j < S; j += NL) {
-               double a = 0.0;
-               for (uint32_t ip = 0; ip < sh.nprm; ip++) {
-                  const uint32_t code = bt.prm[sh.prm_off + ip];
-                  const double kp = __ldg(Ka + (code >> 24)) * __ldg(Kb + ((code >> 16) & 255)) *
-                                    __ldg(Kc + ((code >> 8) & 255)) * __ldg(Kd + (code & 255));
-                  a += kp * bt.AC[(size_t)(sh.prm_off + ip) * S + j];
+            __syncwarp();
+            const double *acp = bt.AC + (size_t)(sh.prm_off + p0) * S;
+            for (int j = lane; j < S; j += 32) {
+               double a = p0 ? ws[j] : 0.0;
+               const double *rp = acp + j;
+               int q = 0;
+               for (; q + 4 <= np; q += 4) {
+                  const double v0 = __ldg(rp), v1 = __ldg(rp + S), v2 = __ldg(rp + 2 * S), v3 = __ldg(rp + 3 * S);
+                  a += kpw[q] * v0;
+                  a += kpw[q + 1] * v1;
+                  a += kpw[q + 2] * v2;
+                  a += kpw[q + 3] * v3;
+                  rp += 4 * S;
                }
-               ws[j * ST] = a;
+               for (; q < np; q++) { a += kpw[q] * __ldg(rp); rp += S; }
+               ws[j] = a;
             }
+            __syncwarp();
          }
-         gsync<NL>();
+         __syncwarp();
          // HRR (reference src/compute_HRR.cpp:7-99), one precompiled instruction per element; the
          // elements of one level are independent, so each lane loads four before it stores any
          for (int lv = 1; lv <= pl->nhlev; lv++) {
@@ -385,26 +358,26 @@ static __device__ __forceinline__ void group_body(const DevCtx &ctx, const Batch
             double R0, R1, R2;
             if (h0.type == 0) { R0 = sh.CD[0]; R1 = sh.CD[1]; R2 = sh.CD[2]; }
             else { R0 = sh.AB[0]; R1 = sh.AB[1]; R2 = sh.AB[2]; }
-            for (int x = x0 + lane; x < x1; x += 4 * NL) {
+            for (int x = x0 + lane; x < x1; x += 4 * 32) {
                uint2 ins[4];
 #pragma unroll
-               for (int u = 0; u < 4; u++) ins[u] = __ldg(&hrec[min(x + u * NL, x1 - 1) - S]);
+               for (int u = 0; u < 4; u++) ins[u] = __ldg(&hrec[min(x + u * 32, x1 - 1) - S]);
                double w1[4], w2[4];
 #pragma unroll
-               for (int u = 0; u < 4; u++) { w1[u] = ws[(ins[u].x & 0x3fffffffu) * ST]; w2[u] = ws[ins[u].y * ST]; }
+               for (int u = 0; u < 4; u++) { w1[u] = ws[ins[u].x & 0x3fffffffu]; w2[u] = ws[ins[u].y]; }
 #pragma unroll
                for (int u = 0; u < 4; u++) {
-                  if (x + u * NL < x1) {
+                  if (x + u * 32 < x1) {
                      const uint32_t dir = ins[u].x >> 30;
                      const double Rd = dir == 0 ? R0 : (dir == 1 ? R1 : R2);
-                     ws[(x + u * NL) * ST] = w1[u] + Rd * w2[u];
+                     ws[x + u * 32] = w1[u] + Rd * w2[u];
                   }
                }
             }
-            gsync<NL>();
+            __syncwarp();
          }
-         for (int x = lane; x < Nc; x += NL) cart[x * ST] += ws[(pl->out_off + x) * ST];
-         gsync<NL>();
+         for (int x = lane; x < Nc; x += 32) cart[x] += ws[pl->out_off + x];
+         __syncwarp();
       }
       // cartesian -> spherical, one centre at a time (a, b, c, d); the two halves of the
       // workspace take turns as the output, and l = 0 centres (a coefficient of 1) are skipped
@@ -415,14 +388,14 @@ static __device__ __forceinline__ void group_body(const DevCtx &ctx, const Batch
          const int ns[4] = {nsa, nsb, nsc, nsd};
          for (int ctr = 0; ctr < 4; ctr++) {
             if (ls[ctr] == 0) continue;
-            double *dst = (sph == ws) ? ws + Nc * ST : ws;
+            double *dst = (sph == ws) ? ws + Nc : ws;
             int npre = 1, npost = 1;
             for (int q = 0; q < ctr; q++) npre *= dims[q];
             for (int q = ctr + 1; q < 4; q++) npost *= dims[q];
-            if (ls[ctr] == 1) sph_pass<1, NL, ST>(sph, dst, npre, npost, lane);
-            else if (ls[ctr] == 2) sph_pass<2, NL, ST>(sph, dst, npre, npost, lane);
-            else sph_pass<3, NL, ST>(sph, dst, npre, npost, lane);
-            gsync<NL>();
+            if (ls[ctr] == 1) sph_pass<1>(sph, dst, npre, npost, lane);
+            else if (ls[ctr] == 2) sph_pass<2>(sph, dst, npre, npost, lane);
+            else sph_pass<3>(sph, dst, npre, npost, lane);
+            __syncwarp();
             dims[ctr] = ns[ctr];
             sph = dst;
          }
@@ -432,7 +405,7 @@ static __device__ __forceinline__ void group_body(const DevCtx &ctx, const Batch
       const double fac = c_symm[k.idx_fac] * ctx.hf_fac;
       const int nscd = nsc * nsd, nsbcd = nsb * nscd;
       const uint32_t Mbcd = (1u << 20) / nsbcd + 1, Mcd = (1u << 20) / nscd + 1, Md = (1u << 20) / nsd + 1;
-      for (int t = lane; t < Ns; t += NL) {
+      for (int t = lane; t < Ns; t += 32) {
          const int isa = div_small(t, Mbcd);
          int rem = t - isa * nsbcd;
          const int isb = div_small(rem, Mcd);
@@ -448,7 +421,7 @@ static __device__ __forceinline__ void group_body(const DevCtx &ctx, const Batch
             atomicOr(ctx.err, 1);
             continue;
          }
-         const double iabcd = -fac * sph[t * ST];
+         const double iabcd = -fac * sph[t];
          for (int sp = 0; sp < ctx.nspin; sp++) {
             const double *Pm = ctx.P[sp];
             double *Km = ctx.K[sp];
@@ -458,7 +431,7 @@ static __device__ __forceinline__ void group_body(const DevCtx &ctx, const Batch
             atomicAdd(Km + Iac, iabcd * __ldg(Pm + Ibd));
          }
       }
-      gsync<NL>();
+      __syncwarp();
    }
 }
 
@@ -501,7 +474,7 @@ __global__ void __launch_bounds__(256, 4) k_group(DevCtx ctx, BatchArgs bt, int 
             gend = G.qrtt_off + (uint32_t)G.nl[0] * G.nl[1] * G.nl[2] * G.nl[3];
          }
          if (bt.gflags && !__ldg(bt.gflags + gi)) continue;   // screened on an incremental replay
-         group_body<32, 1>(ctx, bt, pl, G, q, wbase, wbase + Hws, lane, hrec, kpw, cache, gi);
+         group_body(ctx, bt, pl, G, q, wbase, wbase + Hws, lane, hrec, kpw, cache, gi);
       }
    }
 }
@@ -608,14 +581,6 @@ static int max_dyn_smem() {
    return smax;
 }
 
-int prim_team_size(const ClassPlan &hp) {
-   const int w = hp.V + hp.S;
-   if (w <= 40) return 1;
-   if (w <= 300) return 4;
-   if (w <= 1200) return 8;
-   return 32;
-}
-
 // shared memory of one k_prim2 team, in doubles: cp geometries and (00|00) sums, the pair queue, one
 // batch's Fm, one image's factors and the VRR workspace with its zero
 static size_t prim2_team_doubles(const ClassPlan &hp, int cp) {
@@ -627,6 +592,7 @@ static size_t prim2_team_doubles(const ClassPlan &hp, int cp) {
 // it in many rounds, and too few warps fit an SM to hide them.
 constexpr int kPrim2BlockDoubles = 1500;
 constexpr int kPrim2WideDoubles = 5000;    // and by 256 threads instead of 128 from here on
+int prim_team_size(const ClassPlan &hp) { return hp.V >= kPrim2WideDoubles ? 256 : (hp.V >= kPrim2BlockDoubles ? 128 : 32); }
 
 // Primitive-kernel choice: k_prim3 (generated VRR) for the classes it covers, else k_prim2. Its
 // team is a warp for small workspaces and a block for large ones, and for segments whose chunks are
@@ -647,12 +613,12 @@ cudaError_t launch_prim(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan 
    const size_t plan_bytes = (size_t)plan_smem_doubles() * 8;
    int cp = chunk(148 * 14);
    long nchunk = ((long)bt.nprm + cp - 1) / cp;
-   if (hp.V >= kPrim2BlockDoubles || (hp.V >= 128 && nchunk < 148 * 4)) {
+   if (prim_team_size(hp) > 32 || (hp.V >= 128 && nchunk < 148 * 4)) {
       cp = chunk(148 * 4);
       nchunk = ((long)bt.nprm + cp - 1) / cp;
       const size_t wd = prim2_team_doubles(hp, cp), smem = plan_bytes + wd * 8;
       const unsigned blocks = (unsigned)std::min(nchunk, 148L * 64);
-      if (hp.V >= kPrim2WideDoubles || (hp.V >= 1000 && nchunk < 148)) k_prim2<256><<<blocks, 256, smem, st>>>(ctx, bt, cp, (int)wd);
+      if (prim_team_size(hp) == 256 || (hp.V >= 1000 && nchunk < 148)) k_prim2<256><<<blocks, 256, smem, st>>>(ctx, bt, cp, (int)wd);
       else k_prim2<128><<<blocks, 128, smem, st>>>(ctx, bt, cp, (int)wd);
       return cudaGetLastError();
    }
@@ -669,7 +635,6 @@ size_t group_warp_doubles(const ClassPlan &hp) {
    return (d + 1) & ~(size_t)1;
 }
 
-// returns the number of global-scratch doubles needed (0 if the shared-memory path is used)
 // shared memory ahead of the group kernels' workspaces: the class plan
 static size_t group_hdr_bytes() { return (size_t)plan_smem_doubles() * 8; }
 
@@ -679,6 +644,7 @@ static int group_smem_warps(size_t wd) {
    return std::min(8, (int)(budget / ((wd + kGroupKpDoubles) * 8)));
 }
 
+// doubles of global scratch that k_group needs, and its launch shape there (0: the workspaces fit shared memory)
 size_t group_global_scratch(const ClassPlan &hp, int *grid, int *warps) {
    const size_t wd = group_warp_doubles(hp);
    if (group_smem_warps(wd) >= 1) return 0;
@@ -686,7 +652,6 @@ size_t group_global_scratch(const ClassPlan &hp, int *grid, int *warps) {
    *grid = 148 * 2;
    return wd * (size_t)(*warps) * (*grid);
 }
-
 
 // Group-kernel choice on variant 0: k_group3 (generated HRR, one lane per row) for the classes it
 // covers, k_group_mm (one block per group) for the others; on variant 1 always

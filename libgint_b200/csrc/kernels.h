@@ -80,7 +80,7 @@ size_t group_global_scratch(const ClassPlan &hp, int *grid, int *warps);
 constexpr int kGroupShellCacheDoubles = 16;
 constexpr int kGroupKpDoubles = 32 + kGroupShellCacheDoubles;
 constexpr int kGroupRowsPerWarp = 4;      // consecutive rows a warp of k_group takes at a time
-int prim_team_size(const ClassPlan &hp);
+int prim_team_size(const ClassPlan &hp);   // threads of a k_prim2 team where the segment fills the GPU
 // Incremental replay screening (k_group_screen): mode 0 writes each group's largest |P| over the P
 // blocks its rows read into pmax (the recording's P); mode 1 sets flags[g] = 0 for the groups whose
 // bound * max|dP| / pmax is below eps (current P = dP; max|dP| bounded from the tile maxima tmax of

@@ -430,7 +430,7 @@ static __device__ __forceinline__ SegSum<R> make_segsum(int key, int lane, R *ds
    return sg;
 }
 
-// Nonzero pattern of the cartesian -> spherical rows (bit k of kC2sMask[l][m]: coefficient k of
+// Nonzero pattern of the cartesian -> spherical rows (bit k of c2s_mask(l, m): coefficient k of
 // row m), the integer solid-harmonic rows the coefficients are made from. Terms outside it are
 // exact zeros, so leaving them out changes no sum; upload_constant_tables checks the pattern
 // against the coefficients it uploads.
