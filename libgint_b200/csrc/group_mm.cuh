@@ -188,8 +188,9 @@ static __device__ __forceinline__ int div_nl(int r, int n) {
 // As dense products B T K with precomputed B and K, the HRR and transform of this kernel took five times the
 // operations and up to seven eighths of them on the padding of tiles that shared memory had cut to 1, 2 or
 // 4 rows. Group time of the classes of L = 4..6 and 7..11, kernels one after another, with the products and
-// now: 27.3 and 20.1 ms, 12.4 and 7.3 ms on the 1/4096 sample of the 64-molecule l <= 3 workload; 3.6 and
-// 2.7 ms, 4.2 and 2.5 ms on 24 clusters.
+// now: 27.3 and 20.0 ms, 12.4 and 7.5 ms on the 1/4096 sample of the 64-molecule l <= 3 workload; 3.6 and
+// 2.6 ms, 4.2 and 2.4 ms on 24 clusters. (pp|pp) issues in 52 % of the cycles, its L1 data pipe is 48 % busy,
+// and of 8 warps a scheduler could hold 5 are there, mostly at a barrier (2.7 per issued instruction).
 template <int CLS>
 __global__ void __launch_bounds__(kMmThreads, MmShape<CLS>::MINB) k_group_mm(DevCtx ctx, BatchArgs bt) {
    using Sh = MmShape<CLS>;

@@ -589,14 +589,19 @@ static size_t prim2_team_doubles(const ClassPlan &hp, int cp) {
 }
 
 // A workspace of this many doubles is worked on by a block instead of a warp: a warp takes a level of
-// it in many rounds, and too few warps fit an SM to hide them.
+// it in many rounds, and too few warps fit an SM to hide them. (1/4096 sample of 64 molecules l <= 3, primitive
+// kernels one after another: 39.0 ms with warps only, 38.3; with blocks from 128 doubles on 37.2, but the
+// replay, whose classes overlap, takes 58.2 instead of 57.1 ms. 256 threads from 1500 doubles on: replay 57.9;
+// never: 57.1, there are few primitives of that size.)
 constexpr int kPrim2BlockDoubles = 1500;
 constexpr int kPrim2WideDoubles = 5000;    // and by 256 threads instead of 128 from here on
 int prim_team_size(const ClassPlan &hp) { return hp.V >= kPrim2WideDoubles ? 256 : (hp.V >= kPrim2BlockDoubles ? 128 : 32); }
 
 // Primitive-kernel choice: k_prim3 (generated VRR) for the classes it covers, else k_prim2. Its
 // team is a warp for small workspaces and a block for large ones, and for segments whose chunks are
-// fewer than would give every SM four warps (there one image's chain of levels is the whole time).
+// fewer than would give every SM four warps (there one image's chain of levels is the whole time: 2 molecules
+// and 27 images take 1.60 ms so and 2.19 without, 24 clusters, whose classes fill the GPU beside each other,
+// 4.40 and 4.29; with 128 threads instead of 256 in the larger of these, 1.62 and 4.33).
 cudaError_t launch_prim(const DevCtx &ctx, const BatchArgs &bt, const ClassPlan &hp, cudaStream_t st) {
    if (bt.nprm == 0) return cudaSuccess;
    if (bt.prim_variant == 0 || bt.fp32) {
